@@ -4,14 +4,14 @@
 // transformed by one warp, with no dependencies between TBs; the int16
 // residual goes to the picture's scratch planes (free until SAO runs).
 //
-// k_recon_rows: a persistent kernel in which every warp walks one CTU row at a
+// k_recon_rows: a persistent kernel in which every CTA walks one CTU row at a
 // time. Rows are handed out by an atomic counter, row-major across the
-// pictures of the batch, so a warp only ever waits on the row above, which a
-// running warp took earlier, and the schedule cannot deadlock. Before each CTU
-// the warp waits (bounded) until the row above has finished the CTU
-// above-right of it; the left neighbour is its own previous CTU. It then
-// predicts every coding unit, adds the residual, clips, stores, and publishes
-// the row's progress word.
+// pictures of the batch, so a CTA only ever waits on the row above, which a
+// running CTA took earlier, and the schedule cannot deadlock. Before each CTU
+// it waits (bounded) until the row above has finished the CTU above-right of
+// it; the left neighbour is its own previous CTU. It then predicts every
+// coding unit, adds the residual, clips, stores, and publishes the row's
+// progress word.
 //
 // Follows slice::decode_vvc_frame_picture_with_chroma_qp (slice.rs:4834-4988):
 // predict_coded_block_16 / predict_cclm_with_format_16 prediction (intra.cuh),
@@ -20,7 +20,7 @@
 // clip to 0..2^bd-1. All sums are exact in int32, so reassociating the matrix
 // products (dp2a pairs) gives the reference's results bit for bit.
 #pragma once
-#include "intra.cuh"
+#include "intra_group.cuh"
 #include "vvcg_device.cuh"
 #include "vvcg_tables_dev.cuh"
 
@@ -332,64 +332,122 @@ k_residual(const DevPic* __restrict__ pics, const int16_t* __restrict__ levels, 
   }
 }
 
-// Per-warp shared workspace of the wavefront kernel.
-struct WaveWs {
-  DevPic P;                        // the item's picture, copied once per item
-  IntraWs in[3];                   // prediction state per colour component
-  int16_t luma[32 * 32];           // the CU's reconstructed luma (for CCLM)
+// What the pilot warp prepares of a coding unit, for the whole CTA.
+struct UnitInfo {
+  ModeInfo mode[3];
+  uint8_t resid;   // bit c: component c has a residual
+  uint8_t cclm;    // 1 + CCLM mode, or 0
+  uint8_t ar, bl;  // above-right / below-left samples are coded
+  int16_t gx, gy;
 };
 
-// Luma keeps 2 rows / 5 columns for neighbours and CCLM; chroma 1 / 1.
-constexpr int kLumaRows = 2, kLumaCols = 5, kChromaRows = 1, kChromaCols = 1;
+// Workspace of a reconstruction CTA (one CTU row at a time).
+struct WaveWs {
+  __align__(16) int16_t tile[3][32 * kTilePitch];  // predictions; luma then the reconstruction (for CCLM)
+  DevPic P;                 // the item's picture, copied once per item
+  RawRefs raw[3];           // references per colour component
+  ModeRefs refs[3];
+  CclmRefs cclm;
+  UnitInfo unit[4];         // of units s, s + 1 (and s + 2 while it is prepared), at index s & 3
+  uint32_t item;
+};
 
-// Reconstructs one coding unit in `phase` (0 all samples, 1 the samples other
-// CUs read, 2 the rest). Phase 1 also prepares the prediction state (refs,
-// CCLM models) that phase 2 reuses.
-__device__ void recon_cu(const DevPic& P, const vvcg_cu_rec& rec, int gx, int gy, WaveWs& W, int phase) {
-  const int tb = P.tb;
-  const int bx = gx * tb, by = gy * tb;
-  const uint32_t order = cu_order(P, gx, gy);
-  auto resid = [&](int c, int x0, int y0) -> const int16_t* {
-    return ((rec.cbf >> c) & 1) && rec.level_off[c] >= 0
-               ? reinterpret_cast<const int16_t*>(P.scratch[c]) + (size_t)y0 * P.stride[c] + x0
-               : nullptr;
-  };
-  const int lm = rec.luma_mode <= 69 ? rec.luma_mode : 0;
-  if (phase != 2) prep_intra(P, 0, bx, by, tb, tb, true, lm, order, W.in[0]);
-  emit_intra(P, 0, bx, by, tb, tb, true, lm, W.in[0], resid(0, bx, by), W.luma, phase, kLumaRows,
-             kLumaCols);
-  if (!P.cf) return;
-  const int cxp = bx / P.sub_w, cyp = by / P.sub_h;
-  const int cw = P.tb_cw, ch = P.tb_ch;
+// Warps of a reconstruction CTA: four for luma, kCw for each chroma
+// component, so that every thread has one run of eight samples in the
+// component's largest block (256 samples in 4:2:0, 512 in 4:2:2, 1024 in
+// 4:4:4), then the pilot and the publisher. Registers are given out for
+// multiples of four warps, so at 4:2:0 the last two cost nothing.
+constexpr int kLumaThreads = 128;
+template <int kCw>
+struct ReconShape {
+  static constexpr int kMain = kLumaThreads + 2 * 32 * kCw;
+  static constexpr int kThreads = kMain + 64;
+  static constexpr int kCtasPerSm = kCw == 1 ? 6 : (kCw == 2 ? 5 : 3);
+};
+
+// Barriers of the whole CTA's parts: 4 opens a unit (main warps and pilot), 5
+// closes it (main warps and publisher), 6 is the main warps' own.
+template <int kId>
+__device__ __forceinline__ void part_sync(int n) {
+  asm volatile("bar.sync %0, %1;" ::"n"(kId), "r"(n) : "memory");
+}
+
+// Stores run r of a block (eight samples of a row): clip(prediction +
+// residual) to the plane (`at`: the block's first sample), and with `keep`
+// back to the tile.
+__device__ __forceinline__ void store_run(uint16_t* at, int st, int lw, uint32_t max2, int r, uint4 res, int16_t* tile,
+                                          bool keep) {
+  const int x = 8 * (r & ((1 << (lw - 3)) - 1)), y = r >> (lw - 3);
+  uint4* t = reinterpret_cast<uint4*>(tile + y * kTilePitch + x);
+  uint4 v = *t;
+  v.x = add_clip2(v.x, res.x, max2);
+  v.y = add_clip2(v.y, res.y, max2);
+  v.z = add_clip2(v.z, res.z, max2);
+  v.w = add_clip2(v.w, res.w, max2);
+  *reinterpret_cast<uint4*>(at + y * st + x) = v;
+  if (keep) *t = v;
+}
+
+// Step s of a CTU row (units in z-order inside larger CTUs) on the unit grid.
+__device__ __forceinline__ void row_step(int s, int sh, int cy, int& gx, int& gy) {
+  const int k = s & ((1 << (2 * sh)) - 1);
+  int lx = 0, ly = 0;
+  for (int b = 0; b < sh; b++) {
+    lx |= ((k >> (2 * b)) & 1) << b;
+    ly |= ((k >> (2 * b + 1)) & 1) << b;
+  }
+  gx = ((s >> (2 * sh)) << sh) + lx;
+  gy = (cy << sh) + ly;
+}
+
+// The pilot's unit record: lane c < 3 prepares component c.
+__device__ __forceinline__ void pilot_unit(const DevPic& P, const vvcg_cu_rec& rec, int gx, int gy, int sh,
+                                           UnitInfo& U) {
+  const int lane = threadIdx.x & 31;
   const int chm = rec.chroma_mode;
-  if (chm >= 81 && chm <= 83) {
-    if (phase != 2) prep_cclm(P, cxp, cyp, cw, ch, bx, by, tb, chm - 81, W.in[0], &W.in[1]);
-    for (int c = 1; c <= 2; c++)
-      emit_cclm(P, c, cxp, cyp, cw, ch, bx, by, tb, W.in[0], W.in[c], W.luma, resid(c, cxp, cyp), phase);
-  } else {
-    const int cm = chm <= 69 ? chm : 0;
-    for (int c = 1; c <= 2; c++) {
-      if (phase != 2) prep_intra(P, c, cxp, cyp, cw, ch, false, cm, order, W.in[c]);
-      emit_intra(P, c, cxp, cyp, cw, ch, false, cm, W.in[c], resid(c, cxp, cyp), nullptr, phase,
-                 kChromaRows, kChromaCols);
+  const bool cclm = P.cf && chm >= 81 && chm <= 83;
+  if (lane < 3) {
+    const int mode = lane == 0 ? (rec.luma_mode <= 69 ? rec.luma_mode : 0) : (chm <= 69 ? chm : 0);
+    U.mode[lane] = mode_info(mode, lane ? P.tb_cw : 32, lane ? P.tb_ch : 32, lane == 0);
+  }
+  const bool res = lane < 3 && ((rec.cbf >> lane) & 1) && rec.level_off[lane < 3 ? lane : 0] >= 0;
+  const uint32_t resid = __ballot_sync(0xffffffffu, res);
+  if (lane == 0) {
+    bool ar = gy > 0 && gx + 1 < P.grid_w, bl = false;
+    if (sh) {  // inside larger CTUs the coding order decides
+      const uint32_t order = cu_order(P, gx, gy);
+      ar = ar && cu_order(P, gx + 1, gy - 1) <= order;
+      bl = gx > 0 && gy + 1 < P.grid_h && cu_order(P, gx - 1, gy + 1) <= order;
     }
+    U.resid = (uint8_t)resid;
+    U.cclm = (uint8_t)(cclm ? chm - 80 : 0);
+    U.ar = ar;
+    U.bl = bl;
+    U.gx = (int16_t)gx;
+    U.gy = (int16_t)gy;
   }
 }
 
 // Bounded wait until the CTU row above has finished `need` CTUs in this run
-// (its progress word is (epoch << 32) | count); false when the poll limit ran out.
+// (its progress word is (epoch << 32) | count), which sets `have` to the count
+// seen; false when the poll limit ran out. The first polls follow each other
+// at once (a row mostly waits for a CTU that is about to finish), later ones
+// after growing sleeps.
 __device__ __forceinline__ bool wait_row(const uint64_t* row, uint32_t epoch, uint32_t need,
-                                         uint32_t limit) {
-  uint32_t ns = 64;
+                                         uint32_t limit, uint32_t& have) {
+  uint32_t ns = 32;
   for (uint32_t it = 0;; it++) {
     const uint64_t v = ld_relaxed64(row);
     if ((uint32_t)(v >> 32) == epoch && (uint32_t)v >= need) {
       fence_acq_rel();
+      have = (uint32_t)v;
       return true;
     }
     if (it >= limit) return false;
-    __nanosleep(ns);
-    if (ns < 1024) ns <<= 1;
+    if (it >= 4) {
+      __nanosleep(ns);
+      if (ns < 512) ns <<= 1;
+    }
   }
 }
 
@@ -427,15 +485,17 @@ __device__ __forceinline__ void wavefront_rows(const DevPic* __restrict__ pics, 
       if (above) {
         const uint32_t need = (uint32_t)min(cx + 2, P.ctu_w);
         if (have < need) {
-          int ok = 1;
           if (lane == 0) {
             // once any wait has given up the batch result is void: skip the rest
-            ok = (ld_acquire(status) & kStatusTimeout) == 0 && wait_row(above, epoch, need, spin_limit);
-            if (!ok) atomicOr(status, kStatusTimeout);
+            const bool ok =
+                (ld_acquire(status) & kStatusTimeout) == 0 && wait_row(above, epoch, need, spin_limit, have);
+            if (!ok) {
+              atomicOr(status, kStatusTimeout);
+              have = (uint32_t)P.ctu_w;
+            }
           }
-          ok = __shfl_sync(0xffffffffu, ok, 0);
+          have = __shfl_sync(0xffffffffu, have, 0);
           __syncwarp();
-          have = ok ? need : (uint32_t)P.ctu_w;
         }
       }
       for (int k = 0; k < ncu; k++) {
@@ -454,17 +514,167 @@ __device__ __forceinline__ void wavefront_rows(const DevPic* __restrict__ pics, 
   }
 }
 
-// Reconstruction wavefront over the batch's CTU rows.
-__global__ void __launch_bounds__(kWarpsPerCta * 32, 3)
+// Reconstruction wavefront over the batch's CTU rows: one CTA per CTU row,
+// rows handed out as in wavefront_rows.
+//
+// What bounds it is the serial chain of a picture: CTU x of a row starts when
+// CTU x + 1 of the row above is done, so a picture of W x H CTUs takes at
+// least W + 2 (H - 1) steps, each a poll, one gather round trip, the
+// prediction, the stores and the release of the progress word. A warp per row
+// took 21 us a step; here the 1,536 samples of a unit are spread over 192
+// threads (a run of eight each), a pilot warp prepares the units' modes one
+// step ahead and polls, a publisher warp fences and releases, and the
+// residuals are fetched a step ahead: 3.1 us a step. One 1920x1088 10-bit
+// 4:2:0 picture: 2.41 -> 0.39 ms; 32 of them: 0.74 ms; 128: 5.5 -> 1.9 ms (there
+// the CTAs wait at their barriers, 13 of 25 stall cycles an issue).
+template <int kCw>
+__global__ void __launch_bounds__(ReconShape<kCw>::kThreads, ReconShape<kCw>::kCtasPerSm)
 k_recon_rows(const DevPic* __restrict__ pics, const RowItem* __restrict__ rows, uint32_t n_rows,
              uint32_t* counter, uint32_t epoch, uint32_t spin_limit, uint32_t* status) {
-  extern __shared__ __align__(16) unsigned char wave_smem[];
-  const int wid = threadIdx.x >> 5;
-  WaveWs& W = reinterpret_cast<WaveWs*>(wave_smem)[wid];
+  __shared__ __align__(16) WaveWs W;
+  constexpr int kMain = ReconShape<kCw>::kMain, kThreads = ReconShape<kCw>::kThreads;
+  const int t = threadIdx.x;
   load_cubic_taps();
-  wavefront_rows(pics, rows, n_rows, counter, epoch, spin_limit, status, W, [&](int gx, int gy) {
-    recon_cu(W.P, W.P.cus[gy * W.P.grid_w + gx], gx, gy, W, 0);
-  });
+  for (;;) {
+    __syncthreads();
+    if (t == 0) W.item = atomicAdd(counter, 1u);
+    __syncthreads();
+    if (W.item >= n_rows) break;
+    const RowItem item = rows[W.item];
+    static_assert(sizeof(DevPic) % 4 == 0, "DevPic copy");
+    for (int i = t; i < (int)(sizeof(DevPic) / 4); i += kThreads)
+      reinterpret_cast<uint32_t*>(&W.P)[i] = reinterpret_cast<const uint32_t*>(&pics[item.pic])[i];
+    __syncthreads();
+    const DevPic& P = W.P;
+    const int cy = (int)item.cy;
+    const int sh = P.ctu_log2 - 5;  // units are 32x32
+    const int ncu = 1 << (2 * sh);
+    const int steps = P.ctu_w << (2 * sh);
+    if (t >= kMain + 32) {
+      // ---- publisher: every thread's stores are ordered before the progress
+      // word by the closing barrier and the fence
+      uint64_t* mine = P.row_done + (size_t)cy * kRowFlagStride;
+      for (int s = 0; s < steps; s++) {
+        part_sync<5>(kMain + 32);
+        if (t == kMain + 32 && (s & (ncu - 1)) == ncu - 1) {
+          __threadfence();
+          st_release64(mine, ((uint64_t)epoch << 32) | (uint32_t)((s >> (2 * sh)) + 1));
+        }
+        __syncwarp();
+      }
+    } else if (t >= kMain) {
+      // ---- pilot
+      const uint64_t* above = cy > 0 ? P.row_done + (size_t)(cy - 1) * kRowFlagStride : nullptr;
+      const vvcg_cu_rec* cus = P.cus;
+      const int grid_w = P.grid_w, ctu_w = P.ctu_w;
+      uint32_t have = 0;  // CTUs of the row above known to be finished (lane 0)
+      int gx, gy, nx, ny;
+      row_step(0, sh, cy, gx, gy);
+      pilot_unit(P, cus[gy * grid_w + gx], gx, gy, sh, W.unit[0]);
+      row_step(min(1, steps - 1), sh, cy, nx, ny);
+      vvcg_cu_rec next = cus[ny * grid_w + nx];
+      __syncwarp();
+      part_sync<4>(kMain + 32);  // unit 0 is described
+      for (int s = 0; s < steps; s++) {
+        // unit s + 1 (its record was fetched a step ago)
+        if (s + 1 < steps) {
+          const vvcg_cu_rec rec = next;
+          gx = nx;
+          gy = ny;
+          row_step(min(s + 2, steps - 1), sh, cy, nx, ny);
+          next = cus[ny * grid_w + nx];
+          pilot_unit(P, rec, gx, gy, sh, W.unit[(s + 1) & 3]);
+        }
+        if (t == kMain && above && (s & (ncu - 1)) == 0) {
+          const uint32_t need = (uint32_t)min((s >> (2 * sh)) + 2, ctu_w);
+          // once any wait has given up the batch result is void: skip the rest
+          if (have < need && ((ld_acquire(status) & kStatusTimeout) != 0 ||
+                              !wait_row(above, epoch, need, spin_limit, have))) {
+            atomicOr(status, kStatusTimeout);
+            have = (uint32_t)ctu_w;
+          }
+        }
+        __syncwarp();
+        part_sync<4>(kMain + 32);
+      }
+    } else {
+      // ---- the unit's samples
+      const int comp = t < kLumaThreads ? 0 : 1 + (t - kLumaThreads) / (32 * kCw);
+      const Grp g = comp == 0 ? Grp{t, kLumaThreads, 1} : Grp{(t - kLumaThreads) % (32 * kCw), 32 * kCw, 1 + comp};
+      RawRefs& R = W.raw[comp];
+      ModeRefs& S = W.refs[comp];
+      int16_t* tile = W.tile[comp];
+      const int w = comp ? P.tb_cw : 32, h = comp ? P.tb_ch : 32, lw = ilog2(max(w, 1));
+      const int nruns = (w * h) >> 3;  // 0 without chroma
+      const int st = P.stride[comp], bd = P.bd, cf = P.cf;
+      const uint32_t max2 = ((1u << bd) - 1) * 0x10001u;
+      uint16_t* const plane = P.plane[comp];
+      const int16_t* const scratch = reinterpret_cast<const int16_t*>(P.scratch[comp]);
+      const int nref = 2 * (w + h) + 1;
+      const int ux = w, uy = h;  // a unit's size in the component's samples
+      auto load_res = [&](const UnitInfo& U, int r) -> uint4 {
+        if (!((U.resid >> comp) & 1)) return make_uint4(0, 0, 0, 0);
+        const int x = 8 * (r & ((w >> 3) - 1)), y = r >> (lw - 3);
+        return __ldcs(reinterpret_cast<const uint4*>(scratch + (size_t)(U.gy * uy + y) * st + U.gx * ux + x));
+      };
+      part_sync<4>(kMain + 32);
+      uint4 res = make_uint4(0, 0, 0, 0);
+      if (g.tid < nruns) res = load_res(W.unit[0], g.tid);
+      for (int s = 0; s < steps; s++) {
+        const UnitInfo& U = W.unit[s & 3];
+        const int gx = U.gx, gy = U.gy;
+        const int cclm = U.cclm;
+        uint16_t* const at = plane + (size_t)(gy * uy) * st + gx * ux;
+        RefGeo G{at, st, w, h, 1 << (bd - 1), gy > 0, gx > 0, U.ar != 0, U.bl != 0};
+        const int n = nruns ? nref + (comp == 0 && cclm ? kCclmExtra : 0) : 0;
+        int o[3];
+        bool ok[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          const int e = g.tid + k * g.n;
+          o[k] = e < nref ? ref_offset(G, e) : (e < n ? cclm_offset(G, cf, (gy & ((1 << sh) - 1)) == 0, e - nref) : 0);
+          ok[k] = e < n && o[k] != 0 && (G.ha || G.hl);
+        }
+        part_sync<4>(kMain + 32);
+        // references: at most three loads a thread, all issued before the first is used
+        int v[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) v[k] = ok[k] ? ldp(at + o[k]) : G.def;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          const int e = g.tid + k * g.n;
+          if (e < min(n, nref))
+            ref_put(w, h, e, v[k], R);
+          else if (e < n)
+            cclm_put(e - nref, v[k], W.cclm);
+        }
+        part_sync<6>(kMain);
+        CclmModel M{0, 0, 0};
+        if (comp && cclm) {
+          M = warp_cclm_model(P, gx * 32, gy * 32, w, h, cclm - 1, W.raw[0], W.cclm, R);
+        } else if (nruns) {
+          const ModeInfo m = U.mode[comp];
+          group_prep(g.tid, g.n, m, w, h, R, S);
+          g.sync();
+          const int dc = m.mode == 1 ? warp_dc(R, w, h, (1 << bd) - 1) : 0;
+          for (int r = g.tid; r < nruns; r += g.n) predict_run(r, m, w, h, bd, dc, R, S, tile);
+          g.sync();
+          for (int r = g.tid; r < nruns; r += g.n)
+            store_run(at, st, lw, max2, r, r == g.tid ? res : load_res(U, r), tile, cclm != 0);
+        }
+        if (cclm) {
+          part_sync<6>(kMain);  // the unit's luma is complete
+          if (comp)
+            for (int r = g.tid; r < nruns; r += g.n) {
+              cclm_run(r, cf, bd, gx, lw, M, W.tile[0], W.raw[0], tile);
+              store_run(at, st, lw, max2, r, r == g.tid ? res : load_res(U, r), tile, false);
+            }
+        }
+        part_sync<5>(kMain + 32);
+        if (s + 1 < steps && g.tid < nruns) res = load_res(W.unit[(s + 1) & 3], g.tid);
+      }
+    }
+  }
 }
 
 }  // namespace vvcg

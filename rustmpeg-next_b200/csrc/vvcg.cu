@@ -141,7 +141,7 @@ struct vvcg_ctx {
   std::vector<DbfPass> dbf_ctu;  // CTU-boundary deblocking passes of inter pictures
   DevBuf d_dbf_ctu;
   uint64_t flags_count = 0;
-  int recon_per_sm = 0;  // resident k_recon_rows CTAs per SM
+  int recon_per_sm[3] = {0, 0, 0};  // resident CTAs per SM of each k_recon_rows variant
   // CUDA graph of vvcg_batch_run_graph for the prepared batch and one stage mask
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
@@ -388,6 +388,25 @@ vvcg_status upload_vec(vvcg_ctx* ctx, DevBuf& buf, const std::vector<T>& v) {
   return VVCG_OK;
 }
 
+// The variants of k_recon_rows: chroma warps per component for 256, 512 and
+// 1024 chroma samples a coding unit (4:2:0 and monochrome, 4:2:2, 4:4:4).
+using ReconKernel = void (*)(const DevPic*, const RowItem*, uint32_t, uint32_t*, uint32_t, uint32_t, uint32_t*);
+const ReconKernel kReconKernels[3] = {k_recon_rows<1>, k_recon_rows<2>, k_recon_rows<4>};
+constexpr int kReconThreads[3] = {ReconShape<1>::kThreads, ReconShape<2>::kThreads, ReconShape<4>::kThreads};
+
+int recon_variant(const DevPic& P) {
+  const int n = P.tb_cw * P.tb_ch;
+  return n <= 256 ? 0 : (n <= 512 ? 1 : 2);
+}
+
+cudaError_t recon_occupancy(int per_sm[3]) {
+  for (int v = 0; v < 3; v++) {
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[v], kReconKernels[v], kReconThreads[v], 0);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 bool tu_set_smem_limits();  // every transform-unit kernel variant may use its shared memory
 
 }  // namespace
@@ -422,12 +441,6 @@ vvcg_status vvcg_ctx_create(const vvcg_config* cfg, vvcg_ctx** out) {
     return VVCG_UNAVAILABLE;
   }
   ctx->stream = ctx->own_stream;
-  if (cudaFuncSetAttribute(k_recon_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)(kWarpsPerCta * sizeof(WaveWs))) != cudaSuccess) {
-    cudaStreamDestroy(ctx->own_stream);
-    delete ctx;
-    return VVCG_UNAVAILABLE;
-  }
   if (cudaFuncSetAttribute(k_encode_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)(kEncWarps * sizeof(EncWs))) != cudaSuccess) {
     cudaStreamDestroy(ctx->own_stream);
@@ -445,8 +458,7 @@ vvcg_status vvcg_ctx_create(const vvcg_config* cfg, vvcg_ctx** out) {
     delete ctx;
     return VVCG_UNAVAILABLE;
   }
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->recon_per_sm, k_recon_rows, kWarpsPerCta * 32,
-                                                    kWarpsPerCta * sizeof(WaveWs)) != cudaSuccess) {
+  if (recon_occupancy(ctx->recon_per_sm) != cudaSuccess) {
     cudaStreamDestroy(ctx->own_stream);
     delete ctx;
     return VVCG_UNAVAILABLE;
@@ -811,10 +823,10 @@ vvcg_status enqueue_run(vvcg_ctx* ctx, uint32_t mask, uint32_t epoch, bool clear
     }
     // prediction + reconstruction in CTU wavefront order
     const uint32_t n = (uint32_t)ctx->items.size();
-    const size_t wave_smem = kWarpsPerCta * sizeof(WaveWs);
-    const uint32_t warps = (uint32_t)ctx->num_sms * std::max(1, ctx->recon_per_sm) * kWarpsPerCta;
-    const uint32_t grid = (std::min<uint32_t>(n, warps) + kWarpsPerCta - 1) / kWarpsPerCta;
-    k_recon_rows<<<grid, kWarpsPerCta * 32, wave_smem, ctx->stream>>>(
+    int v = 0;  // the picture with the most chroma decides
+    for (auto& P : ctx->pics) v = std::max(v, recon_variant(P));
+    const uint32_t grid = std::min<uint32_t>(n, (uint32_t)(ctx->num_sms * std::max(1, ctx->recon_per_sm[v])));
+    kReconKernels[v]<<<grid, kReconThreads[v], 0, ctx->stream>>>(
         (const DevPic*)ctx->d_pics.p, (const RowItem*)ctx->d_items.p, n, ctrl, epoch, ctx->spin_limit, ctrl + 1);
     CK(cudaGetLastError(), "recon launch");
     (*launches)++;
@@ -2652,7 +2664,7 @@ struct StaticDevice {
   bool ready = false;
   unsigned char* scratch = nullptr;  // device address of g_static_scratch
   int num_sms = 0;
-  int recon_ctas_per_sm = 0;
+  int recon_per_sm[3] = {0, 0, 0};
 };
 
 constexpr int kStaticMaxDevices = 64;
@@ -2689,15 +2701,10 @@ vvcg_status static_setup(int dev, const StaticDevice** out, char* err, size_t er
     tables_ctx.device = dev;
     if (upload_tables(&tables_ctx) != VVCG_OK)
       return static_fail(err, err_cap, VVCG_UNAVAILABLE, "%s", tables_ctx.err.c_str());
-    const int wave_smem = (int)(kWarpsPerCta * sizeof(WaveWs));
-    SCK(cudaFuncSetAttribute(k_recon_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, wave_smem),
-        "cudaFuncSetAttribute");
     void* p = nullptr;
     SCK(cudaGetSymbolAddress(&p, g_static_scratch), "cudaGetSymbolAddress");
     SCK(cudaDeviceGetAttribute(&S.num_sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
-    SCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&S.recon_ctas_per_sm, k_recon_rows,
-                                                      kWarpsPerCta * 32, wave_smem),
-        "occupancy");
+    SCK(recon_occupancy(S.recon_per_sm), "occupancy");
     S.scratch = (unsigned char*)p;
     S.ready = true;
   }
@@ -2844,10 +2851,10 @@ extern "C" vvcg_status vvcg_recon_picture_static(const vvcg_pic_desc* pic, const
         d_pic, levels, num_levels, ctrl + 1);
     SCK(cudaGetLastError(), "residual (TU tools) launch");
   }
-  const uint32_t warps = (uint32_t)S->num_sms * std::max(1, S->recon_ctas_per_sm) * kWarpsPerCta;
-  const uint32_t grid = (std::min<uint32_t>((uint32_t)P.ctu_h, warps) + kWarpsPerCta - 1) / kWarpsPerCta;
+  const int v = recon_variant(P);
+  const uint32_t grid = std::min<uint32_t>((uint32_t)P.ctu_h, (uint32_t)(S->num_sms * std::max(1, S->recon_per_sm[v])));
   const uint32_t epoch = 1;  // progress lines were cleared above
-  k_recon_rows<<<grid, kWarpsPerCta * 32, kWarpsPerCta * sizeof(WaveWs), s>>>(
+  kReconKernels[v]<<<grid, kReconThreads[v], 0, s>>>(
       d_pic, d_rows, (uint32_t)P.ctu_h, ctrl, epoch, kDefaultSpinLimit, ctrl + 1);
   SCK(cudaGetLastError(), "recon launch");
   for (int k = 0; k < 4; k++) {
