@@ -400,34 +400,6 @@ __device__ __forceinline__ void row_step(int s, int sh, int cy, int& gx, int& gy
   gy = (cy << sh) + ly;
 }
 
-// The pilot's unit record: lane c < 3 prepares component c.
-__device__ __forceinline__ void pilot_unit(const DevPic& P, const vvcg_cu_rec& rec, int gx, int gy, int sh,
-                                           UnitInfo& U) {
-  const int lane = threadIdx.x & 31;
-  const int chm = rec.chroma_mode;
-  const bool cclm = P.cf && chm >= 81 && chm <= 83;
-  if (lane < 3) {
-    const int mode = lane == 0 ? (rec.luma_mode <= 69 ? rec.luma_mode : 0) : (chm <= 69 ? chm : 0);
-    U.mode[lane] = mode_info(mode, lane ? P.tb_cw : 32, lane ? P.tb_ch : 32, lane == 0);
-  }
-  const bool res = lane < 3 && ((rec.cbf >> lane) & 1) && rec.level_off[lane < 3 ? lane : 0] >= 0;
-  const uint32_t resid = __ballot_sync(0xffffffffu, res);
-  if (lane == 0) {
-    bool ar = gy > 0 && gx + 1 < P.grid_w, bl = false;
-    if (sh) {  // inside larger CTUs the coding order decides
-      const uint32_t order = cu_order(P, gx, gy);
-      ar = ar && cu_order(P, gx + 1, gy - 1) <= order;
-      bl = gx > 0 && gy + 1 < P.grid_h && cu_order(P, gx - 1, gy + 1) <= order;
-    }
-    U.resid = (uint8_t)resid;
-    U.cclm = (uint8_t)(cclm ? chm - 80 : 0);
-    U.ar = ar;
-    U.bl = bl;
-    U.gx = (int16_t)gx;
-    U.gy = (int16_t)gy;
-  }
-}
-
 // Bounded wait until the CTU row above has finished `need` CTUs in this run
 // (its progress word is (epoch << 32) | count), which sets `have` to the count
 // seen; false when the poll limit ran out. The first polls follow each other
@@ -451,71 +423,55 @@ __device__ __forceinline__ bool wait_row(const uint64_t* row, uint32_t epoch, ui
   }
 }
 
-// The CTU-row wavefront, shared by reconstruction and encoding: one warp per
-// CTU row. Rows are handed out by an atomic counter row-major across the
-// pictures of the batch, so a warp only ever waits on the row above, which a
-// running warp took earlier, and the schedule cannot deadlock. Walking its row
-// left to right, the warp codes a CTU once the row above has finished the CTU
-// above-right of it (or the last CTU of the row), then publishes its own
-// progress. The left neighbour is the warp's own previous CTU, so only the row
-// above needs synchronisation. `cu(gx, gy)` codes one CU with W.P set.
-template <class Ws, class CuFn>
-__device__ __forceinline__ void wavefront_rows(const DevPic* __restrict__ pics, const RowItem* __restrict__ rows,
-                                               uint32_t n_rows, uint32_t* counter, uint32_t epoch,
-                                               uint32_t spin_limit, uint32_t* status, Ws& W, CuFn&& cu) {
+// The pilot's wait before a CTU: the row above has finished `need` CTUs.
+__device__ __forceinline__ void pilot_wait(const uint64_t* above, uint32_t epoch, int need, int ctu_w,
+                                           uint32_t spin_limit, uint32_t* status, uint32_t& have) {
+  // once any wait has given up the batch result is void: skip the rest
+  if (have < (uint32_t)need && ((ld_acquire(status) & kStatusTimeout) != 0 ||
+                                !wait_row(above, epoch, (uint32_t)need, spin_limit, have))) {
+    atomicOr(status, kStatusTimeout);
+    have = (uint32_t)ctu_w;
+  }
+}
+
+// Whether the samples above-right (ar) and below-left (bl) of a unit are
+// coded before it.
+__device__ __forceinline__ void unit_edges(const DevPic& P, int gx, int gy, int sh, bool& ar, bool& bl) {
+  ar = gy > 0 && gx + 1 < P.grid_w;
+  bl = false;
+  if (sh) {  // inside larger CTUs the coding order decides
+    const uint32_t order = cu_order(P, gx, gy);
+    ar = ar && cu_order(P, gx + 1, gy - 1) <= order;
+    bl = gx > 0 && gy + 1 < P.grid_h && cu_order(P, gx - 1, gy + 1) <= order;
+  }
+}
+
+// The pilot's unit record: lane c < 3 prepares component c.
+__device__ __forceinline__ void pilot_unit(const DevPic& P, const vvcg_cu_rec& rec, int gx, int gy, int sh,
+                                           UnitInfo& U) {
   const int lane = threadIdx.x & 31;
-  for (;;) {
-    uint32_t it = 0;
-    if (lane == 0) it = atomicAdd(counter, 1u);
-    it = __shfl_sync(0xffffffffu, it, 0);
-    if (it >= n_rows) break;
-    const RowItem item = rows[it];
-    static_assert(sizeof(DevPic) % 4 == 0 && sizeof(DevPic) <= 64 * 4, "DevPic copy");
-    for (int i = lane; i < (int)(sizeof(DevPic) / 4); i += 32)
-      reinterpret_cast<uint32_t*>(&W.P)[i] = reinterpret_cast<const uint32_t*>(&pics[item.pic])[i];
-    __syncwarp();
-    const DevPic& P = W.P;
-    const int cy = (int)item.cy;
-    const int sh = P.ctu_log2 - ilog2(P.tb);
-    const int ncu = 1 << (2 * sh);
-    const uint64_t* above = cy > 0 ? P.row_done + (size_t)(cy - 1) * kRowFlagStride : nullptr;
-    uint64_t* mine = P.row_done + (size_t)cy * kRowFlagStride;
-    uint32_t have = 0;  // CTUs of the row above known to be finished
-    for (int cx = 0; cx < P.ctu_w; cx++) {
-      if (above) {
-        const uint32_t need = (uint32_t)min(cx + 2, P.ctu_w);
-        if (have < need) {
-          if (lane == 0) {
-            // once any wait has given up the batch result is void: skip the rest
-            const bool ok =
-                (ld_acquire(status) & kStatusTimeout) == 0 && wait_row(above, epoch, need, spin_limit, have);
-            if (!ok) {
-              atomicOr(status, kStatusTimeout);
-              have = (uint32_t)P.ctu_w;
-            }
-          }
-          have = __shfl_sync(0xffffffffu, have, 0);
-          __syncwarp();
-        }
-      }
-      for (int k = 0; k < ncu; k++) {
-        int lx = 0, ly = 0;
-        for (int b = 0; b < sh; b++) {
-          lx |= ((k >> (2 * b)) & 1) << b;
-          ly |= ((k >> (2 * b + 1)) & 1) << b;
-        }
-        cu((cx << sh) + lx, (cy << sh) + ly);
-      }
-      // publish: every lane's stores are ordered before the progress word
-      __threadfence();
-      __syncwarp();
-      if (lane == 0) st_release64(mine, ((uint64_t)epoch << 32) | (uint32_t)(cx + 1));
-    }
+  const int chm = rec.chroma_mode;
+  const bool cclm = P.cf && chm >= 81 && chm <= 83;
+  if (lane < 3) {
+    const int mode = lane == 0 ? (rec.luma_mode <= 69 ? rec.luma_mode : 0) : (chm <= 69 ? chm : 0);
+    U.mode[lane] = mode_info(mode, lane ? P.tb_cw : 32, lane ? P.tb_ch : 32, lane == 0);
+  }
+  const bool res = lane < 3 && ((rec.cbf >> lane) & 1) && rec.level_off[lane < 3 ? lane : 0] >= 0;
+  const uint32_t resid = __ballot_sync(0xffffffffu, res);
+  if (lane == 0) {
+    bool ar, bl;
+    unit_edges(P, gx, gy, sh, ar, bl);
+    U.resid = (uint8_t)resid;
+    U.cclm = (uint8_t)(cclm ? chm - 80 : 0);
+    U.ar = ar;
+    U.bl = bl;
+    U.gx = (int16_t)gx;
+    U.gy = (int16_t)gy;
   }
 }
 
 // Reconstruction wavefront over the batch's CTU rows: one CTA per CTU row,
-// rows handed out as in wavefront_rows.
+// rows handed out in order (row-major across the pictures) by an atomic counter.
 //
 // What bounds it is the serial chain of a picture: CTU x of a row starts when
 // CTU x + 1 of the row above is done, so a picture of W x H CTUs takes at
@@ -585,15 +541,8 @@ k_recon_rows(const DevPic* __restrict__ pics, const RowItem* __restrict__ rows, 
           next = cus[ny * grid_w + nx];
           pilot_unit(P, rec, gx, gy, sh, W.unit[(s + 1) & 3]);
         }
-        if (t == kMain && above && (s & (ncu - 1)) == 0) {
-          const uint32_t need = (uint32_t)min((s >> (2 * sh)) + 2, ctu_w);
-          // once any wait has given up the batch result is void: skip the rest
-          if (have < need && ((ld_acquire(status) & kStatusTimeout) != 0 ||
-                              !wait_row(above, epoch, need, spin_limit, have))) {
-            atomicOr(status, kStatusTimeout);
-            have = (uint32_t)ctu_w;
-          }
-        }
+        if (t == kMain && above && (s & (ncu - 1)) == 0)
+          pilot_wait(above, epoch, min((s >> (2 * sh)) + 2, ctu_w), ctu_w, spin_limit, status, have);
         __syncwarp();
         part_sync<4>(kMain + 32);
       }

@@ -442,7 +442,7 @@ vvcg_status vvcg_ctx_create(const vvcg_config* cfg, vvcg_ctx** out) {
   }
   ctx->stream = ctx->own_stream;
   if (cudaFuncSetAttribute(k_encode_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)(kEncWarps * sizeof(EncWs))) != cudaSuccess) {
+                           (int)sizeof(EncWs)) != cudaSuccess) {
     cudaStreamDestroy(ctx->own_stream);
     delete ctx;
     return VVCG_UNAVAILABLE;
@@ -2423,12 +2423,10 @@ extern "C" vvcg_status vvcg_encode_batch(vvcg_ctx* ctx, const vvcg_pic_desc* pic
   CK(cudaMemsetAsync(ctrl, 0, 2 * sizeof(uint32_t), ctx->stream), "memset");
   ctx->epoch++;
   const uint32_t n = (uint32_t)ctx->items.size();
-  const size_t smem = kEncWarps * sizeof(EncWs);
   int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_encode_rows, kEncWarps * 32, smem), "occupancy");
-  const uint32_t warps = (uint32_t)ctx->num_sms * std::max(1, per_sm) * kEncWarps;
-  const uint32_t grid = (std::min<uint32_t>(n, warps) + kEncWarps - 1) / kEncWarps;
-  k_encode_rows<<<grid, kEncWarps * 32, smem, ctx->stream>>>((const DevPic*)ctx->d_pics.p,
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_encode_rows, kEncThreads, sizeof(EncWs)), "occupancy");
+  const uint32_t grid = std::min<uint32_t>(n, (uint32_t)(ctx->num_sms * std::max(1, per_sm)));
+  k_encode_rows<<<grid, kEncThreads, sizeof(EncWs), ctx->stream>>>((const DevPic*)ctx->d_pics.p,
                                                             (const RowItem*)ctx->d_items.p, n, ctrl, ctx->epoch,
                                                             ctx->spin_limit, ctrl + 1);
   CK(cudaGetLastError(), "encode launch");
