@@ -450,7 +450,7 @@ vvcg_status gen_enqueue(vvcg_ctx* ctx, uint32_t* n) {
     const uint32_t cnt = G.tu_count[bin];
     if (cnt) {
       const TuVariant& V = kTuTable[bin][ctx->tu_pick[0][bin]];
-      V.inv<<<(cnt + V.warps - 1) / V.warps, V.warps * 32, V.smem, ctx->stream>>>(
+      V.inv<<<(cnt + V.warps - 1) / V.warps, V.warps * 32, V.smem_inv, ctx->stream>>>(
           (const vvcg_tu_rec*)G.tus.p, (const uint32_t*)G.tu_idx.p + first, cnt, (const int16_t*)G.levels.p,
           (int16_t*)G.res.p);
       CK(cudaGetLastError(), "residual launch");

@@ -119,8 +119,8 @@ __device__ void p_predict_component(const PPicDev& P, const vvcg_inter_cu& rec, 
 // then add, clip and store.
 __global__ void __launch_bounds__(kPWarps * 32, 7)
 k_p_cu(const PPicDev* __restrict__ pics, const int16_t* __restrict__ levels, uint64_t n_levels, uint32_t* status) {
-  __shared__ __align__(16) int32_t ws_luma[2][1024 + kTuPad];     // the luma warp's transform tiles
-  __shared__ __align__(16) int32_t ws_chroma[2][2][256 + kTuPad];  // the chroma warps' tiles
+  __shared__ __align__(16) int16_t ws_luma[tu_inv_ws(1024)];     // the luma warp's transform tiles
+  __shared__ __align__(16) int16_t ws_chroma[2][tu_inv_ws(256)];  // the chroma warps' tiles
   __shared__ __align__(16) PMcSmem mc;
   __shared__ __align__(16) int16_t res[1024 + 2 * 256];
   __shared__ __align__(16) int16_t pred[1024 + 2 * 256];
@@ -160,9 +160,7 @@ k_p_cu(const PPicDev* __restrict__ pics, const int16_t* __restrict__ levels, uin
         t.flags = ts ? VVCG_TU_TRANSFORM_SKIP : ((P.flags & 1) ? VVCG_TU_DEP_QUANT : 0);
         t.mts_idx = t.lfnst_idx = t.lfnst_mode = 0;
         t.in_off = t.out_off = 0;
-        int32_t* A = c ? ws_chroma[c - 1][0] : ws_luma[0];
-        int32_t* B = c ? ws_chroma[c - 1][1] : ws_luma[1];
-        warp_tu_inverse(t, src, r, A, B, lane);
+        warp_tu_inverse(t, src, r, c ? ws_chroma[c - 1] : ws_luma, lane);
       }
     }
     if (!coded)

@@ -353,6 +353,34 @@ vvcg_status upload_tables(vvcg_ctx* ctx) {
       pos += build_scan(1 << a, 1 << b, tu_scans.data() + pos);
     }
   if (pos != kTuScanTotal) return fail(ctx, VVCG_EXECUTION, "scan table size %d", pos);
+  std::vector<int16_t> tu_pos(kTuScanTotal, 0);
+  for (int a = 0; a <= 6; a++)
+    for (int b = 0; b <= 6; b++) {
+      const int o = tu_offs[a * 7 + b], w = 1 << a, tw = std::min(w, 32), n = tw * std::min(1 << b, 32);
+      for (int k = 0; k < n; k++) {
+        const int r = tu_scans[o + k];
+        tu_pos[o + (r / w) * tw + r % w] = (int16_t)k;
+      }
+    }
+  CK(cudaMemcpyToSymbol(g_tu_scan_pos, tu_pos.data(), sizeof(int16_t) * kTuScanTotal), "tables");
+  // packed matrix rows of both directions (tu_mat_row)
+  std::vector<uint32_t> tm(kTmWords, 0);
+  uint16_t tm_off[2][3][7] = {};
+  int tm_at = 0;
+  for (int dir = 0; dir < 2; dir++)
+    for (int type = 0; type < 3; type++)
+      for (int lg = type ? 2 : 1; lg <= (type ? 5 : 6); lg++) {
+        const int n = 1 << lg, words = std::max(1, n / 4);
+        const int8_t* m = type == 0 ? d2[lg - 1] : (type == 1 ? s7[lg - 2] : c8[lg - 2]);
+        if (tm_at + n * words > kTmWords) return fail(ctx, VVCG_EXECUTION, "matrix table size");
+        tm_off[dir][type][lg] = (uint16_t)tm_at;
+        int8_t* row = reinterpret_cast<int8_t*>(tm.data() + tm_at);
+        for (int o = 0; o < n; o++, row += 4 * words)
+          for (int k = 0; k < n; k++) row[k] = dir ? m[k * n + o] : m[o * n + k];
+        tm_at += (n * words + 3) & ~3;
+      }
+  CK(cudaMemcpyToSymbol(g_tm, tm.data(), sizeof(uint32_t) * tm_at), "tables");
+  CK(cudaMemcpyToSymbol(c_tm_off, tm_off, sizeof(tm_off)), "tables");
   CK(cudaMemcpyToSymbol(g_tu_scan, tu_scans.data(), sizeof(int16_t) * pos), "tables");
   CK(cudaMemcpyToSymbol(g_tu_scan_off, tu_offs, sizeof(tu_offs)), "tables");
   CK(cudaMemcpyToSymbol(g_lfnst8, kLfnst8x8, sizeof(kLfnst8x8)), "tables");
@@ -2456,12 +2484,13 @@ using TuKernel = void (*)(const vvcg_tu_rec*, const uint32_t*, uint32_t, const i
 struct TuVariant {
   TuKernel inv, fwd;
   int warps;
-  size_t smem;
+  size_t smem_inv, smem_fwd;
 };
 constexpr int kTuBins = 3, kTuVariants = 3;
 template <int kEl, int kW>
 TuVariant tu_variant() {
-  return TuVariant{k_tu<kEl, kW, false>, k_tu<kEl, kW, true>, kW, tu_smem_bytes<kEl, kW>()};
+  return TuVariant{k_tu<kEl, kW, false>, k_tu<kEl, kW, true>, kW, tu_smem_bytes<kEl, kW>(false),
+                   tu_smem_bytes<kEl, kW>(true)};
 }
 const TuVariant kTuTable[kTuBins][kTuVariants] = {
     {tu_variant<256, 2>(), tu_variant<256, 4>(), tu_variant<256, 8>()},
@@ -2473,8 +2502,8 @@ bool tu_set_smem_limits() {
   for (int b = 0; b < kTuBins; b++)
     for (int v = 0; v < kTuVariants; v++) {
       const TuVariant& V = kTuTable[b][v];
-      if (cudaFuncSetAttribute(V.inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)V.smem) != cudaSuccess ||
-          cudaFuncSetAttribute(V.fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)V.smem) != cudaSuccess)
+      if (cudaFuncSetAttribute(V.inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)V.smem_inv) != cudaSuccess ||
+          cudaFuncSetAttribute(V.fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)V.smem_fwd) != cudaSuccess)
         return false;
     }
   return true;
@@ -2539,7 +2568,7 @@ vvcg_status tu_launch(vvcg_ctx* ctx, const uint32_t count[kTuBins], int b, int v
   uint32_t first = 0;
   for (int k = 0; k < b; k++) first += count[k];
   const TuKernel k = forward ? V.fwd : V.inv;
-  k<<<(count[b] + V.warps - 1) / V.warps, V.warps * 32, V.smem, ctx->stream>>>(
+  k<<<(count[b] + V.warps - 1) / V.warps, V.warps * 32, forward ? V.smem_fwd : V.smem_inv, ctx->stream>>>(
       (const vvcg_tu_rec*)ctx->d_tu_recs.p, (const uint32_t*)ctx->d_tu_idx.p + first, count[b], in, out);
   CK(cudaGetLastError(), "transform-unit launch");
   ctx->launches++;
