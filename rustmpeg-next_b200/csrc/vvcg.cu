@@ -1168,7 +1168,8 @@ static vvcg_status mc_common(vvcg_ctx* ctx, const uint16_t* ref, uint32_t w, uin
     return fail(ctx, VVCG_INVALID_INPUT, "invalid MC arguments");
   if (n == 0) return VVCG_OK;
   McParams pm{ref, nullptr, (int32_t)w, (int32_t)h, (int32_t)stride, bd, chroma};
-  k_mc<<<n, 256, 0, ctx->stream>>>(pm, blocks, n, out, (uint32_t*)ctx->d_ctrl.p + 1);
+  (chroma ? k_mc<4, false> : k_mc<8, false>)<<<dim3((n + kMcWarps - 1) / kMcWarps, kMcSplit), kMcWarps * 32, 0, ctx->stream>>>(
+      pm, blocks, n, out);
   CK(cudaGetLastError(), "mc launch");
   ctx->launches++;
   return VVCG_OK;
@@ -1181,7 +1182,8 @@ static vvcg_status mc_common_8(vvcg_ctx* ctx, const uint8_t* ref, uint32_t w, ui
     return fail(ctx, VVCG_INVALID_INPUT, "invalid MC arguments");
   if (n == 0) return VVCG_OK;
   McParams pm{nullptr, ref, (int32_t)w, (int32_t)h, (int32_t)stride, 8, chroma};
-  k_mc<<<n, 256, 0, ctx->stream>>>(pm, blocks, n, out, (uint32_t*)ctx->d_ctrl.p + 1);
+  (chroma ? k_mc<4, true> : k_mc<8, true>)<<<dim3((n + kMcWarps - 1) / kMcWarps, kMcSplit), kMcWarps * 32, 0, ctx->stream>>>(
+      pm, blocks, n, out);
   CK(cudaGetLastError(), "mc launch");
   ctx->launches++;
   return VVCG_OK;
@@ -1216,7 +1218,7 @@ vvcg_status vvcg_mc_bi_average_16_dev(vvcg_ctx* ctx, const int32_t* p0, const in
   if (!p0 || !p1 || !out || bd < 8 || bd > 12 || bcw > 4)
     return fail(ctx, VVCG_INVALID_INPUT, "invalid bi-average arguments");
   if (!count) return VVCG_OK;
-  uint32_t grid = (uint32_t)std::min<uint64_t>((count + 255) / 256, (uint64_t)ctx->num_sms * 16);
+  uint32_t grid = (uint32_t)std::min<uint64_t>((count + 1023) / 1024, (uint64_t)ctx->num_sms * 16);
   k_bi_average<<<grid, 256, 0, ctx->stream>>>(p0, p1, count, bcw, bd, out);
   CK(cudaGetLastError(), "bi average launch");
   ctx->launches++;

@@ -10,14 +10,14 @@ namespace vvcg {
 __constant__ int c_ang_table[32];
 __constant__ int c_inv_ang_table[32];
 __constant__ int c_intra_filter_thr[8];
-__constant__ int8_t c_chroma_taps4[128];
+__constant__ __align__(8) int8_t c_chroma_taps4[128];  // also read as packed words
 __constant__ uint8_t c_cclm_div_sig[16];
 __constant__ int c_inv_quant_scale[2][6];
 __constant__ int c_quant_scale[2][6];
 __constant__ int16_t c_dbf_tc[66];
 __constant__ int16_t c_dbf_beta[64];
-__constant__ int8_t c_luma_taps8[128];
-__constant__ int8_t c_affine_taps8[128];
+__constant__ __align__(8) int8_t c_luma_taps8[128];
+__constant__ __align__(8) int8_t c_affine_taps8[128];
 __constant__ int c_luma_alt_hpel[8];
 __constant__ int c_bcw_weights[5];
 __constant__ int c_alf_clip[3][4];
