@@ -1,13 +1,8 @@
-// Luma intra mode searches on the GPU.
-//
-// 1. The 8-bit multi-tool encoder's decision: choose_luma_intra_pred_mode
-//    (crates/rustmpeg-video/src/vvc/predict.rs:2737-2801) over Planar, DC and
-//    the 65 angular modes (or the 6 MPMs), then the encoder's MRL candidates
-//    (slice.rs:2698-2731): reference lines 1 and 2 for mpm[1..5]. Cost: SAD.
-// 2. The CTU full search of the GPU encoder: every block of the six split
-//    types of a 32x32 CTU, each over the 67 modes (or a candidate list), on
-//    8..12-bit samples with the predictors of predict_block_16
-//    (predict.rs:3079-3410), cost = 8x8 Hadamard SATD + lambda * mode bits.
+// Luma intra mode search of the 8-bit multi-tool encoder:
+// choose_luma_intra_pred_mode (crates/rustmpeg-video/src/vvc/predict.rs:
+// 2737-2801) over Planar, DC and the 65 angular modes (or the 6 MPMs), then the
+// encoder's MRL candidates (slice.rs:2698-2731): reference lines 1 and 2 for
+// mpm[1..5]. Cost: SAD.
 //
 // One CTA per block, one warp per candidate at a time; each warp builds the
 // candidate's extended reference arrays in its own shared buffers exactly as
@@ -25,7 +20,6 @@ constexpr int kIsrWarps = 8;
 constexpr int kIsrRow = 136;  // 2 * 64 + 3 + 4 + 1: longest MRL row
 constexpr int kIsrBuf = 520;  // base + 2 max(w, h) + 2 max(refW, refH) + 64 for 64x64 (516)
 constexpr int kIsrMaxCand = 67 + 10;
-constexpr int kSatdMaxSamples = 1024;
 
 // init_angular_params (predict.rs:1608-1685) for a luma w x h block without
 // ISP and reference line mri.
@@ -76,7 +70,6 @@ __device__ __forceinline__ Ang8 ang8_params(int dir, int w, int h, int mri) {
   return p;
 }
 
-template <bool kSatd>
 struct IsrShared {
   uint16_t src[64 * 64];
   // reference rows as MrlRefSamples: [set][0 above / 1 left]; sets 0 / 1 are
@@ -87,14 +80,13 @@ struct IsrShared {
   int16_t tl[2];
   int32_t dc;
   uint32_t cost[kIsrMaxCand];
-  int16_t buf[kIsrWarps][2][kIsrBuf];                               // a warp's ref_above / ref_left
-  int16_t res[kSatd ? kIsrWarps : 1][kSatd ? kSatdMaxSamples : 1];  // a warp's residual block
+  int16_t buf[kIsrWarps][2][kIsrBuf];  // a warp's ref_above / ref_left
 };
 
 // Calls sink(i, v) with the prediction v of every sample i (raster) of a w x h
 // block for one angular candidate (predict_angular_with_params_bd), by one warp.
-template <bool kSatd, typename Sink>
-__device__ void isr_angular(IsrShared<kSatd>& S, int warp, int lane, int w, int h, int dir, int set, int mri, int bd,
+template <typename Sink>
+__device__ void isr_angular(IsrShared& S, int warp, int lane, int w, int h, int dir, int set, int mri, int bd,
                             Sink sink) {
   const Ang8 P = ang8_params(dir, w, h, mri);
   const int def = 1 << (bd - 1), maxv = (1 << bd) - 1;
@@ -187,8 +179,8 @@ __device__ void isr_angular(IsrShared<kSatd>& S, int warp, int lane, int w, int 
 }
 
 // Planar (predict.rs:1688-1719) or DC (:1722-1736) with PDPC (:1739-1754).
-template <bool kSatd, typename Sink>
-__device__ void isr_planar_dc(IsrShared<kSatd>& S, int lane, int w, int h, bool planar, Sink sink) {
+template <typename Sink>
+__device__ void isr_planar_dc(IsrShared& S, int lane, int w, int h, bool planar, Sink sink) {
   const int f = (planar && w * h > 32) ? 1 : 0;  // uses_reference_filter for luma Planar
   const int16_t* top = S.ref[f][0];
   const int16_t* left = S.ref[f][1];
@@ -215,8 +207,8 @@ __device__ void isr_planar_dc(IsrShared<kSatd>& S, int lane, int w, int h, bool 
 // at 8..12 bits), RefSamples::filtered (:1233-1267), the line-0 rows
 // (MrlRefSamples::from_ref_samples, :1058-1075) and the DC value. With
 // `mrl`, also lines 1 and 2 (gather_references_mrl, :1141-1231).
-template <bool kSatd, typename T>
-__device__ void isr_prepare(IsrShared<kSatd>& S, const T* rec, int64_t rs, int width, int height, int bx, int by,
+template <typename T>
+__device__ void isr_prepare(IsrShared& S, const T* rec, int64_t rs, int width, int height, int bx, int by,
                             int w, int h, int bd, bool mrl, bool ctu_top) {
   const int t = threadIdx.x;
   const int def = 1 << (bd - 1);
@@ -318,7 +310,7 @@ struct IsrArgs {
 };
 
 __global__ void __launch_bounds__(kIsrWarps * 32) k_luma_intra_search_8(const __grid_constant__ IsrArgs A) {
-  __shared__ IsrShared<false> S;
+  __shared__ IsrShared S;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   for (int q = blockIdx.x; q < A.n; q += gridDim.x) {
     const vvcg_intra_search_req R = A.reqs[q];
@@ -377,174 +369,6 @@ __global__ void __launch_bounds__(kIsrWarps * 32) k_luma_intra_search_8(const __
     }
     __syncthreads();
   }
-}
-
-// ------------------------------------------------------- CTU full search ----
-
-// Bits a block is charged in the search cost: a header of 8 bits (split
-// flags, cbf and the like) plus its mode, ordered by the default MPM list
-// (derive_intra_mpms with no neighbours, predict.rs): MPM i costs 2 + i bits,
-// any other mode 7.
-__device__ __forceinline__ int search_mode_bits(int m) {
-  return 8 + (m == 0 ? 2 : m == 1 ? 3 : m == 50 ? 4 : m == 18 ? 5 : m == 46 ? 6 : 7);
-}
-
-// One block of one split type of one CTU.
-struct CostReq {
-  uint32_t x, y;
-  uint8_t log2_w, log2_h, n_cand, reserved;
-  uint8_t cand[6];
-  uint16_t slot;  // block slot of the CTU, 0..14
-  uint32_t ctu;   // index of the CTU request
-};
-
-struct CostArgs {
-  const uint16_t* src;
-  int64_t stride;
-  int32_t width, height, bd, n;
-  uint32_t lambda_q8;
-  const CostReq* reqs;
-  uint32_t* block_cost;  // [ctu][15]
-  uint8_t* block_mode;   // [ctu][15]
-  uint32_t* mode_costs;  // optional [ctu][67]: every mode's cost of the unsplit CU (slot 0, full set)
-};
-
-// 8x8 Hadamard SATD of a w x h residual block (w, h multiples of 8) in the
-// warp's buffer: each 8-lane group transforms one 8x8 tile (rows, then
-// columns); a tile's SATD is (sum |coefficient| + 2) >> 2.
-__device__ __forceinline__ uint32_t satd8x8_warp(int16_t* res, int lane, int w, int h) {
-  const int tiles = (w >> 3) * (h >> 3);
-  const int g = lane >> 3, r = lane & 7;
-  uint32_t total = 0;
-  for (int t0 = 0; t0 < tiles; t0 += 4) {
-    const int tile = t0 + g;
-    const bool act = tile < tiles;
-    const int tx = act ? (tile % (w >> 3)) * 8 : 0, ty = act ? (tile / (w >> 3)) * 8 : 0;
-    int v[8];
-    if (act) {
-#pragma unroll
-      for (int k = 0; k < 8; k++) v[k] = res[(ty + r) * w + tx + k];
-      // 8-point Hadamard of row r
-#pragma unroll
-      for (int s = 1; s < 8; s <<= 1)
-#pragma unroll
-        for (int k = 0; k < 8; k++)
-          if (!(k & s)) {
-            const int a = v[k], b = v[k + s];
-            v[k] = a + b;
-            v[k + s] = a - b;
-          }
-    }
-    // rows back to the buffer, then each lane takes column r of its tile
-    if (act) {
-#pragma unroll
-      for (int k = 0; k < 8; k++) res[(ty + r) * w + tx + k] = (int16_t)v[k];
-    }
-    __syncwarp();
-    int col[8];
-    if (act) {
-#pragma unroll
-      for (int k = 0; k < 8; k++) col[k] = res[(ty + k) * w + tx + r];
-    }
-    __syncwarp();
-    uint32_t s_abs = 0;
-    if (act) {
-#pragma unroll
-      for (int s = 1; s < 8; s <<= 1)
-#pragma unroll
-        for (int k = 0; k < 8; k++)
-          if (!(k & s)) {
-            const int a = col[k], b = col[k + s];
-            col[k] = a + b;
-            col[k + s] = a - b;
-          }
-#pragma unroll
-      for (int k = 0; k < 8; k++) s_abs += (uint32_t)abs(col[k]);
-    }
-    // the tile's sum over its 8 lanes
-    s_abs += __shfl_xor_sync(0xFFFFFFFFu, s_abs, 1);
-    s_abs += __shfl_xor_sync(0xFFFFFFFFu, s_abs, 2);
-    s_abs += __shfl_xor_sync(0xFFFFFFFFu, s_abs, 4);
-    if (act && r == 0) total += (s_abs + 2) >> 2;
-  }
-  return __reduce_add_sync(0xFFFFFFFFu, total);
-}
-
-__global__ void __launch_bounds__(kIsrWarps * 32) k_cost_search(const __grid_constant__ CostArgs A) {
-  __shared__ IsrShared<true> S;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  for (int q = blockIdx.x; q < A.n; q += gridDim.x) {
-    const CostReq R = A.reqs[q];
-    if (R.log2_w == 0) continue;  // an unused slot (pruned search)
-    const int w = 1 << R.log2_w, h = 1 << R.log2_h, bx = (int)R.x, by = (int)R.y;
-    for (int i = t; i < w * h; i += blockDim.x) S.src[i] = A.src[(int64_t)(by + i / w) * A.stride + bx + (i % w)];
-    isr_prepare(S, A.src, A.stride, A.width, A.height, bx, by, w, h, A.bd, false, true);
-    const int n_cand = R.n_cand ? R.n_cand : 67;
-    int16_t* res = S.res[warp];
-    for (int c = warp; c < n_cand; c += kIsrWarps) {
-      const int mode = R.n_cand ? R.cand[c] : c;
-      auto put = [&](int i, int v) { res[i] = (int16_t)((int)S.src[i] - v); };
-      if (mode <= 1)
-        isr_planar_dc(S, lane, w, h, mode == 0, put);
-      else
-        isr_angular(S, warp, lane, w, h, mode, (ang8_params(mode, w, h, 0).ref_filter) ? 1 : 0, 0, A.bd, put);
-      __syncwarp();
-      const uint32_t satd = satd8x8_warp(res, lane, w, h);
-      __syncwarp();
-      if (lane == 0) S.cost[c] = satd + (uint32_t)(((uint64_t)A.lambda_q8 * search_mode_bits(mode)) >> 8);
-    }
-    __syncthreads();
-    if (t == 0) {
-      uint32_t best = 0xFFFFFFFFu;
-      int bm = 0;
-      for (int c = 0; c < n_cand; c++)
-        if (S.cost[c] < best) {
-          best = S.cost[c];
-          bm = R.n_cand ? R.cand[c] : c;
-        }
-      A.block_cost[(size_t)R.ctu * 15 + R.slot] = best;
-      A.block_mode[(size_t)R.ctu * 15 + R.slot] = (uint8_t)bm;
-    }
-    if (A.mode_costs && R.slot == 0 && R.n_cand == 0)
-      for (int c = t; c < 67; c += blockDim.x) A.mode_costs[(size_t)R.ctu * 67 + c] = S.cost[c];
-    __syncthreads();
-  }
-}
-
-// Slots of the 15 blocks of a 32x32 CTU per split type and the split bits.
-__constant__ uint8_t c_split_first[6] = {0, 1, 5, 7, 9, 12};
-__constant__ uint8_t c_split_count[6] = {1, 4, 2, 2, 3, 3};
-__constant__ uint8_t c_split_bits[6] = {1, 2, 3, 3, 4, 4};
-
-// Per CTU: each evaluated split's cost (its blocks' costs + lambda * split
-// bits), the first lowest wins.
-__global__ void k_ctu_search_combine(const vvcg_ctu_search_req* reqs, int n, uint32_t lambda_q8,
-                                     const uint32_t* block_cost, const uint8_t* block_mode,
-                                     vvcg_ctu_search_res* out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t mask = reqs[i].split_mask;
-  vvcg_ctu_search_res o;
-  o.cost = 0xFFFFFFFFu;
-  o.split = 0xFF;
-  o.cu_mode = 0xFF;
-  for (int k = 0; k < 4; k++) o.modes[k] = 0xFF;
-  o.reserved[0] = o.reserved[1] = 0;
-  for (int s = 0; s < 6; s++) {
-    o.split_cost[s] = 0xFFFFFFFFu;
-    if (!(mask & (1u << s))) continue;
-    uint64_t c = ((uint64_t)lambda_q8 * c_split_bits[s]) >> 8;
-    for (int k = 0; k < c_split_count[s]; k++) c += block_cost[(size_t)i * 15 + c_split_first[s] + k];
-    o.split_cost[s] = c < 0xFFFFFFFEull ? (uint32_t)c : 0xFFFFFFFEu;
-    if (o.split_cost[s] < o.cost) {
-      o.cost = o.split_cost[s];
-      o.split = (uint8_t)s;
-      for (int k = 0; k < 4; k++)
-        o.modes[k] = k < c_split_count[s] ? block_mode[(size_t)i * 15 + c_split_first[s] + k] : 0xFF;
-    }
-  }
-  if (mask & 1u) o.cu_mode = block_mode[(size_t)i * 15];
-  out[i] = o;
 }
 
 }  // namespace vvcg

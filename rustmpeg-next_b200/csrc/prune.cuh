@@ -1,23 +1,18 @@
 // CNN-pruned CTU search: the pruner's logits choose, per CTU, the intra
 // candidates (the top_modes most probable modes) and the split types (the
-// top_splits most probable) that the full search of intra_search.cuh then
+// top_splits most probable) that the full search of ctu_search.cuh then
 // evaluates; a head whose chosen candidates hold less than the threshold of
 // its softmax probability mass (for a calibrated network: the chance that
 // the full search's choice is among them), or under the max-probability
 // rule whose most probable entry is below the threshold, keeps its full set
 // (all 67 modes / all 6 splits). Everything
 // stays on the device: requests are built from the logits by one thread per
-// CTU and expanded into the 15 block slots of the search.
+// CTU.
 #pragma once
 #include "cnn.cuh"
-#include "intra_search.cuh"
+#include "ctu_search.cuh"
 
 namespace vvcg {
-
-// Positions of the 15 blocks of a 32x32 CTU (x, y, log2 w, log2 h) by slot.
-__constant__ uint8_t c_search_blocks[15][4] = {
-    {0, 0, 5, 5},  {0, 0, 4, 4},  {16, 0, 4, 4}, {0, 16, 4, 4}, {16, 16, 4, 4}, {0, 0, 5, 4},  {0, 16, 5, 4}, {0, 0, 4, 5},
-    {16, 0, 4, 5}, {0, 0, 5, 3},  {0, 8, 5, 4},  {0, 24, 5, 3}, {0, 0, 3, 5},   {8, 0, 4, 5},  {24, 0, 3, 5}};
 
 // indices of the k largest of v[0..n) (ties: the lower index first)
 __device__ __forceinline__ void top_k(const float* v, int n, int k, uint8_t* out) {
@@ -45,7 +40,7 @@ __device__ __forceinline__ float top_mass(const float* v, int n, const uint8_t* 
 
 __global__ void k_prune_requests(const float* __restrict__ logits, const uint32_t* __restrict__ xy, int n, int width,
                                  int height, int top_modes, int top_splits, float thr, bool max_prob,
-                                 vvcg_ctu_search_req* reqs, CostReq* blocks) {
+                                 vvcg_ctu_search_req* reqs) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   vvcg_ctu_search_req r{};
@@ -70,24 +65,6 @@ __global__ void k_prune_requests(const float* __restrict__ logits, const uint32_
     }
   }
   reqs[i] = r;
-  for (int s = 0; s < 6; s++) {
-    const int first = c_split_first[s], count = c_split_count[s];
-    for (int k = 0; k < count; k++) {
-      const int slot = first + k;
-      CostReq b{};
-      if (r.split_mask & (1u << s)) {
-        b.x = r.x + c_search_blocks[slot][0];
-        b.y = r.y + c_search_blocks[slot][1];
-        b.log2_w = c_search_blocks[slot][2];
-        b.log2_h = c_search_blocks[slot][3];
-        b.n_cand = r.n_cand;
-        for (int c = 0; c < 6; c++) b.cand[c] = r.cand[c];
-      }  // else log2_w = 0: the slot is skipped
-      b.slot = (uint16_t)slot;
-      b.ctu = (uint32_t)i;
-      blocks[(size_t)i * 15 + slot] = b;
-    }
-  }
 }
 
 }  // namespace vvcg

@@ -19,6 +19,7 @@
 #include "enc.cuh"
 #include "filters.cuh"
 #include "gen_intra.cuh"
+#include "ctu_search.cuh"
 #include "intra_search.cuh"
 #include "inter_search.cuh"
 #include "inter_tools.cuh"
@@ -134,7 +135,7 @@ struct vvcg_ctx {
   uint8_t tu_pick[2][3] = {{1, 1, 1}, {1, 1, 1}};
   DevBuf d_lmcs;  // a device copy of the LMCS tables of the last call
   DevBuf d_alfp, d_alfc;  // general-decoder ALF parameters and CTU switches
-  DevBuf d_search_reqs, d_search_cost, d_search_mode, d_search_ctus;  // CTU full search
+  DevBuf d_search_cost, d_search_mode, d_search_ctus;  // CTU full search
   DevBuf d_cnn_pack, d_cnn_packT;  // packed bf16 convolution weights of the CNN (forward / transposed)
   DevBuf d_cnn_acts, d_cnn_logits, d_cnn_gap, d_cnn_partial;  // CNN training workspace
   DevBuf d_me_reqs, d_me_cands;  // motion-estimation requests and merge candidates
@@ -522,7 +523,7 @@ void vvcg_ctx_destroy(vvcg_ctx* ctx) {
                     &ctx->d_dbf[1], &ctx->d_dbf[2], &ctx->d_dbf[3], &ctx->d_sao, &ctx->d_alf, &ctx->d_sao_alf, &ctx->d_tmaps,
                     &ctx->d_cus, &ctx->d_levels, &ctx->d_ctus, &ctx->d_aps, &ctx->d_ctrl,
                     &ctx->d_tu_recs, &ctx->d_tu_idx, &ctx->d_lmcs, &ctx->d_alfp, &ctx->d_alfc,
-                    &ctx->d_search_reqs, &ctx->d_search_cost, &ctx->d_search_mode, &ctx->d_search_ctus,
+                    &ctx->d_search_cost, &ctx->d_search_mode, &ctx->d_search_ctus,
                     &ctx->d_cnn_pack, &ctx->d_cnn_packT, &ctx->d_cnn_acts, &ctx->d_cnn_logits, &ctx->d_cnn_gap,
                     &ctx->d_cnn_partial, &ctx->d_me_reqs, &ctx->d_me_cands, &ctx->d_dbf_ctu})
     b->release();
@@ -1598,17 +1599,21 @@ extern "C" vvcg_status vvcg_inter_search_8_dev(vvcg_ctx* ctx, const uint8_t* src
 // ---------------------------------------------------------------------------
 // CTU full search of the GPU encoder (vvcg_ctu_search_dev).
 // ---------------------------------------------------------------------------
-// Blocks of a 32x32 CTU: (x, y, log2 w, log2 h) per slot; the slots of split
-// s are c_split_first[s] .. + c_split_count[s] - 1.
-static const uint8_t kSearchBlocks[15][4] = {
-    {0, 0, 5, 5},                                                   // none
-    {0, 0, 4, 4},  {16, 0, 4, 4}, {0, 16, 4, 4}, {16, 16, 4, 4},    // quad
-    {0, 0, 5, 4},  {0, 16, 5, 4},                                   // binary, horizontal split
-    {0, 0, 4, 5},  {16, 0, 4, 5},                                   // binary, vertical split
-    {0, 0, 5, 3},  {0, 8, 5, 4},  {0, 24, 5, 3},                    // ternary, horizontal split
-    {0, 0, 3, 5},  {8, 0, 4, 5},  {24, 0, 3, 5}};                   // ternary, vertical split
-static const uint8_t kSearchSplitFirst[6] = {0, 1, 5, 7, 9, 12};
-static const uint8_t kSearchSplitCount[6] = {1, 4, 2, 2, 3, 3};
+static vvcg_status ctu_search_launch(vvcg_ctx* ctx, const uint16_t* src, uint64_t stride, uint32_t width,
+                                     uint32_t height, uint8_t bit_depth, uint32_t lambda_q8, uint32_t num_ctus,
+                                     vvcg_ctu_search_res* res, uint32_t* mode_costs) {
+  CtsArgs A{src, (int64_t)stride, (int32_t)width, (int32_t)height, bit_depth, lambda_q8,
+            (const vvcg_ctu_search_req*)ctx->d_search_ctus.p, (uint32_t*)ctx->d_search_cost.p,
+            (uint8_t*)ctx->d_search_mode.p, mode_costs};
+  k_ctu_costs<<<num_ctus * 6, kCtsWarps * 32, 0, ctx->stream>>>(A);
+  CK(cudaGetLastError(), "search launch");
+  k_ctu_search_combine<<<(num_ctus + 127) / 128, 128, 0, ctx->stream>>>(
+      (const vvcg_ctu_search_req*)ctx->d_search_ctus.p, (int)num_ctus, lambda_q8,
+      (const uint32_t*)ctx->d_search_cost.p, (const uint8_t*)ctx->d_search_mode.p, res);
+  CK(cudaGetLastError(), "search launch");
+  ctx->launches += 2;
+  return VVCG_OK;
+}
 
 extern "C" vvcg_status vvcg_ctu_search_dev(vvcg_ctx* ctx, const uint16_t* src, uint64_t stride, uint32_t width,
                                            uint32_t height, uint8_t bit_depth, uint32_t lambda_q8,
@@ -1621,8 +1626,6 @@ extern "C" vvcg_status vvcg_ctu_search_dev(vvcg_ctx* ctx, const uint16_t* src, u
   if (bit_depth < 8 || bit_depth > 12) return fail(ctx, VVCG_INVALID_INPUT, "bit depth");
   if (width > (1u << 20) || height > (1u << 20)) return fail(ctx, VVCG_LIMIT_EXCEEDED, "plane larger than 2^20");
   if (num_reqs > (1u << 24)) return fail(ctx, VVCG_LIMIT_EXCEEDED, "more than 2^24 CTUs");
-  std::vector<CostReq> blocks;
-  blocks.reserve((size_t)num_reqs * 15);
   for (uint32_t i = 0; i < num_reqs; i++) {
     const vvcg_ctu_search_req& q = reqs[i];
     if ((uint64_t)q.x + 32 > width || (uint64_t)q.y + 32 > height)
@@ -1631,47 +1634,16 @@ extern "C" vvcg_status vvcg_ctu_search_dev(vvcg_ctx* ctx, const uint16_t* src, u
     if (q.n_cand > 6) return fail(ctx, VVCG_INVALID_INPUT, "request %u: more than 6 candidates", i);
     for (int k = 0; k < q.n_cand; k++)
       if (q.cand[k] > 66) return fail(ctx, VVCG_INVALID_INPUT, "request %u: candidate %d is not a mode", i, k);
-    for (int sp = 0; sp < 6; sp++) {
-      if (!(q.split_mask & (1u << sp))) continue;
-      for (int k = 0; k < kSearchSplitCount[sp]; k++) {
-        const int slot = kSearchSplitFirst[sp] + k;
-        CostReq b{};
-        b.x = q.x + kSearchBlocks[slot][0];
-        b.y = q.y + kSearchBlocks[slot][1];
-        b.log2_w = kSearchBlocks[slot][2];
-        b.log2_h = kSearchBlocks[slot][3];
-        b.n_cand = q.n_cand;
-        for (int c = 0; c < 6; c++) b.cand[c] = q.cand[c];
-        b.slot = (uint16_t)slot;
-        b.ctu = i;
-        blocks.push_back(b);
-      }
-    }
   }
   CK(cudaSetDevice(ctx->device), "cudaSetDevice");
-  CK(ctx->d_search_reqs.reserve(sizeof(CostReq) * blocks.size()), "cudaMalloc");
   CK(ctx->d_search_ctus.reserve(sizeof(vvcg_ctu_search_req) * num_reqs), "cudaMalloc");
   CK(ctx->d_search_cost.reserve(sizeof(uint32_t) * 15 * (size_t)num_reqs), "cudaMalloc");
   CK(ctx->d_search_mode.reserve(15 * (size_t)num_reqs), "cudaMalloc");
   // pageable sources: the copies have read them when cudaMemcpyAsync returns
-  CK(cudaMemcpyAsync(ctx->d_search_reqs.p, blocks.data(), sizeof(CostReq) * blocks.size(), cudaMemcpyHostToDevice,
-                     ctx->stream),
-     "upload");
   CK(cudaMemcpyAsync(ctx->d_search_ctus.p, reqs, sizeof(vvcg_ctu_search_req) * num_reqs, cudaMemcpyHostToDevice,
                      ctx->stream),
      "upload");
-  CostArgs A{src, (int64_t)stride, (int32_t)width, (int32_t)height, bit_depth, (int32_t)blocks.size(), lambda_q8,
-             (const CostReq*)ctx->d_search_reqs.p, (uint32_t*)ctx->d_search_cost.p,
-             (uint8_t*)ctx->d_search_mode.p};
-  const uint32_t grid = (uint32_t)std::min<size_t>(blocks.size(), (size_t)ctx->num_sms * 8);
-  k_cost_search<<<grid, kIsrWarps * 32, 0, ctx->stream>>>(A);
-  CK(cudaGetLastError(), "search launch");
-  k_ctu_search_combine<<<(num_reqs + 127) / 128, 128, 0, ctx->stream>>>(
-      (const vvcg_ctu_search_req*)ctx->d_search_ctus.p, (int)num_reqs, lambda_q8,
-      (const uint32_t*)ctx->d_search_cost.p, (const uint8_t*)ctx->d_search_mode.p, res);
-  CK(cudaGetLastError(), "search launch");
-  ctx->launches += 2;
-  return VVCG_OK;
+  return ctu_search_launch(ctx, src, stride, width, height, bit_depth, lambda_q8, num_reqs, res, nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -1725,25 +1697,15 @@ static vvcg_status ctu_search_xy(vvcg_ctx* ctx, const uint16_t* src, uint64_t st
     return fail(ctx, VVCG_LIMIT_EXCEEDED, "plane or CTU count too large");
   CK(cudaSetDevice(ctx->device), "cudaSetDevice");
   const size_t nb = (size_t)num_ctus * 15;
-  CK(ctx->d_search_reqs.reserve(sizeof(CostReq) * nb), "cudaMalloc");
   CK(ctx->d_search_ctus.reserve(sizeof(vvcg_ctu_search_req) * num_ctus), "cudaMalloc");
   CK(ctx->d_search_cost.reserve(sizeof(uint32_t) * nb), "cudaMalloc");
   CK(ctx->d_search_mode.reserve(nb), "cudaMalloc");
   k_prune_requests<<<(num_ctus + 127) / 128, 128, 0, ctx->stream>>>(
       logits, ctu_xy, (int)num_ctus, (int)width, (int)height, (int)top_modes, (int)top_splits, threshold,
-      rule == VVCG_PRUNE_MAX_PROB, (vvcg_ctu_search_req*)ctx->d_search_ctus.p, (CostReq*)ctx->d_search_reqs.p);
+      rule == VVCG_PRUNE_MAX_PROB, (vvcg_ctu_search_req*)ctx->d_search_ctus.p);
   CK(cudaGetLastError(), "prune launch");
-  CostArgs A{src, (int64_t)stride, (int32_t)width, (int32_t)height, bit_depth, (int32_t)nb, lambda_q8,
-             (const CostReq*)ctx->d_search_reqs.p, (uint32_t*)ctx->d_search_cost.p,
-             (uint8_t*)ctx->d_search_mode.p, mode_costs};
-  k_cost_search<<<(uint32_t)std::min<size_t>(nb, (size_t)ctx->num_sms * 8), kIsrWarps * 32, 0, ctx->stream>>>(A);
-  CK(cudaGetLastError(), "search launch");
-  k_ctu_search_combine<<<(num_ctus + 127) / 128, 128, 0, ctx->stream>>>(
-      (const vvcg_ctu_search_req*)ctx->d_search_ctus.p, (int)num_ctus, lambda_q8,
-      (const uint32_t*)ctx->d_search_cost.p, (const uint8_t*)ctx->d_search_mode.p, res);
-  CK(cudaGetLastError(), "search launch");
-  ctx->launches += 3;
-  return VVCG_OK;
+  ctx->launches++;
+  return ctu_search_launch(ctx, src, stride, width, height, bit_depth, lambda_q8, num_ctus, res, mode_costs);
 }
 
 // ---------------------------------------------------------------------------
