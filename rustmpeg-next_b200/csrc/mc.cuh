@@ -95,9 +95,11 @@ struct McWs {
 // One tile of a block by one warp: outputs tw x th at o (row pitch bw), whose
 // window starts at plane position (wx0, wy0). False, with nothing written,
 // when a sample of the window lies above the bit depth.
-template <int kTaps, bool kEight>
+// Out: int32_t (the interpolation calls) or int16_t (predictions kept in
+// shared memory).
+template <int kTaps, bool kEight, class Out>
 __device__ __forceinline__ bool mc_tile(const McParams& Pm, const McFilter& F, int wx0, int wy0, int tw, int th,
-                                        int32_t* o, int bw, McWs& S, int lane) {
+                                        Out* o, int bw, McWs& S, int lane) {
   constexpr int half = kTaps / 2 - 1;
   const int ww = tw + kTaps - 1, wh = th + kTaps - 1;
   // the window, at column `xo` of its rows; groups of four samples where the
@@ -166,10 +168,10 @@ __device__ __forceinline__ bool mc_tile(const McParams& Pm, const McFilter& F, i
 #pragma unroll
         for (int k = 0; k < 8; k++) v[k] = mc_1d(F, v[k]);
       }
-      int32_t* d = o + (size_t)y * bw + x0;
+      Out* d = o + (size_t)y * bw + x0;
 #pragma unroll
       for (int k = 0; k < 8; k++)
-        if (x0 + k < tw) d[k] = v[k];
+        if (x0 + k < tw) d[k] = (Out)v[k];
     }
     __syncwarp();
     return true;
@@ -192,7 +194,7 @@ __device__ __forceinline__ bool mc_tile(const McParams& Pm, const McFilter& F, i
   __syncwarp();
   // columns: two by four outputs a lane and step
   const int cp = (tw + 1) >> 1;
-  const bool pair = ((reinterpret_cast<uintptr_t>(o) & 7) | (bw & 1)) == 0;
+  const bool pair = ((reinterpret_cast<uintptr_t>(o) & (2 * sizeof(Out) - 1)) | (bw & 1)) == 0;
   const int crows = per_warp(cp), cy = div_lane(lane, cp), x = 2 * (lane - cy * cp);
   for (int y0 = cy < crows ? 4 * cy : th; y0 < th; y0 += 4 * crows) {
     constexpr int kRows = kTaps + 3;
@@ -221,12 +223,15 @@ __device__ __forceinline__ bool mc_tile(const McParams& Pm, const McFilter& F, i
     for (int q = 0; q < 4; q++) {
       if (y0 + q >= th) continue;
       const int va = F.fx == 0 ? mc_1d(F, a[q]) : mc_2d(F, a[q]), vb = F.fx == 0 ? mc_1d(F, b[q]) : mc_2d(F, b[q]);
-      int32_t* d = o + (size_t)(y0 + q) * bw + x;
+      Out* d = o + (size_t)(y0 + q) * bw + x;
       if (pair && x + 1 < tw) {
-        *reinterpret_cast<int2*>(d) = make_int2(va, vb);
+        if constexpr (sizeof(Out) == 4)
+          *reinterpret_cast<int2*>(d) = make_int2(va, vb);
+        else
+          *reinterpret_cast<uint32_t*>(d) = __byte_perm((uint32_t)va, (uint32_t)vb, 0x5410);
       } else {
-        d[0] = va;
-        if (x + 1 < tw) d[1] = vb;
+        d[0] = (Out)va;
+        if (x + 1 < tw) d[1] = (Out)vb;
       }
     }
   }

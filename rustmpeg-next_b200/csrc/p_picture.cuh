@@ -9,10 +9,9 @@
 // (reconstruct_component_full, slice.rs:1920: DCT-2 or transform skip,
 // regular or dependent dequantisation) and the clipped sum. Every CTU of a
 // picture depends only on the reference pictures, so one CTA per CTU runs
-// them all at once: warp 0 turns the Y levels into the residual (the TU
-// path's warp_tu_inverse) while warps 1 and 2 do Cb and Cr and then, with
-// warp 3, stage each component's reference window and filter it into a
-// prediction in shared memory; all four warps then store the clipped sums
+// them all at once: the TU path's warp_tu_inverse turns the levels into
+// residuals and the interpolation's tiles (mc.cuh) predict into shared memory;
+// all four warps then store the clipped sums
 // into the picture's buffer slot. apply_inter_loop_filters'
 // CTU-boundary deblocking (slice.rs:2291) follows for pictures that enable
 // it. Pictures are grouped into levels by their slots (a picture waits for
@@ -32,118 +31,109 @@ struct PPicDev {
   uint32_t flags;  // bit0 dependent quantisation, bit1 sparse levels
 };
 
-// The MC window of one component (the luma 39 x 39, or chroma 19 x 19) and
-// the horizontal pass's rows. 16 bits suffice: samples are 8-bit and the
-// horizontal sums of the 8-tap / 4-tap filters stay within +-32767.
-struct PMcSmem {
-  int16_t win[39][40];
-  int16_t tmp[39][32];
-};
+// A component's reference plane and the unit's filter for it (the 8-bit
+// functions' rounding on 16-bit planes).
+template <bool kLuma>
+__device__ __forceinline__ McParams p_params(const PPicDev& P, const vvcg_inter_cu& rec, int comp) {
+  return McParams{P.ref[min((int)rec.ref_idx[0], P.num_refs - 1)][comp], nullptr, kLuma ? P.w : P.w / 2,
+                  kLuma ? P.h : P.h / 2, P.stride[comp], 8, kLuma ? 0 : 1};
+}
+template <bool kLuma>
+__device__ __forceinline__ McFilter p_filter(const McParams& Pm, const vvcg_inter_cu& rec) {
+  vvcg_mc_block B;
+  B.mv_x = rec.mv[0][0];
+  B.mv_y = rec.mv[0][1];
+  B.flags = kLuma && (rec.flags & VVCG_INTER_CU_ALT_HPEL) ? VVCG_MC_ALT_HPEL : 0;
+  return mc_filter<true>(Pm, B);
+}
 
-// Barrier of warps 1..3, the prediction warps of a CTA.
-__device__ __forceinline__ void p_mc_sync() { asm volatile("bar.sync 1, 96;" ::: "memory"); }
-
-// The inter prediction of one component of a coding unit into `pred` (int16,
-// n x n raster), by the prediction warps (thread `tid` of 96).
-__device__ void p_predict_component(const PPicDev& P, const vvcg_inter_cu& rec, int comp, int bx, int by,
-                                    int16_t* __restrict__ pred, PMcSmem& S, int tid) {
-  constexpr int nth = 96;
-  const bool luma = comp == 0;
-  const int n = luma ? 32 : 16, ntap = luma ? 8 : 4, half = luma ? 3 : 1;
-  const int pw = luma ? P.w : P.w / 2, ph = luma ? P.h : P.h / 2;
-  const int x0 = luma ? bx : bx / 2, y0 = luma ? by : by / 2;
-  const int rstride = P.stride[comp];
-  const bool has = (rec.inter_dir & 1) && rec.ref_idx[0] >= 0;
-  if (!has) {  // predict_inter_pu without a usable list: 128
-    for (int i = tid; i < n * n; i += nth) pred[i] = 128;
-    return;
-  }
-  const uint16_t* ref = P.ref[min((int)rec.ref_idx[0], P.num_refs - 1)][comp];
-  // 1/16-sample luma motion; 4:2:0 chroma reads it as 1/32 of a chroma sample
-  const int mx = rec.mv[0][0], my = rec.mv[0][1];
-  const int dx = luma ? mx >> 4 : mx >> 5, dy = luma ? my >> 4 : my >> 5;
-  const int fx = luma ? mx & 15 : mx & 31, fy = luma ? my & 15 : my & 31;
-  const bool alt = (rec.flags & VVCG_INTER_CU_ALT_HPEL) != 0;
-  int fh[8], fv[8];
-  for (int k = 0; k < ntap; k++) {
-    if (luma) {
-      fh[k] = (alt && fx == 8) ? c_luma_alt_hpel[k] : c_luma_taps8[fx * 8 + k];
-      fv[k] = (alt && fy == 8) ? c_luma_alt_hpel[k] : c_luma_taps8[fy * 8 + k];
+// A prediction tile whose reference window holds samples above 8 bits (a
+// picture-buffer upload does not reject them), one output at a time with the
+// 16-bit window and intermediate the filters then wrap in.
+template <bool kLuma>
+__device__ __noinline__ void p_tile_wide(const PPicDev* pic, const vvcg_inter_cu* unit, int comp, int bx, int by,
+                                         int16_t* o) {
+  constexpr int tw = kLuma ? 32 : 16, ntap = kLuma ? 8 : 4, half = ntap / 2 - 1;
+  const int lane = threadIdx.x & 31;
+  const McParams Pm = p_params<kLuma>(*pic, *unit, comp);
+  const McFilter F = p_filter<kLuma>(Pm, *unit);
+  const int wx0 = bx + F.dx - half, wy0 = by + F.dy - half;
+  auto at = [&](int x, int y) -> int {
+    return (int16_t)Pm.ref[(size_t)clampi(wy0 + y, 0, Pm.h - 1) * Pm.stride + clampi(wx0 + x, 0, Pm.w - 1)];
+  };
+  for (int i = lane; i < tw * 16; i += 32) {
+    const int x = i % tw, y = i / tw;
+    int s = 0;
+    if (F.fx == 0 && F.fy == 0) {
+      s = at(x + half, y + half);
+    } else if (F.fy == 0) {
+      for (int k = 0; k < ntap; k++) s += mc_tap(F.th0, F.th1, k) * at(x + k, y + half);
+      s = clampi((s + 32) >> 6, 0, 255);
+    } else if (F.fx == 0) {
+      for (int k = 0; k < ntap; k++) s += mc_tap(F.tv0, F.tv1, k) * at(x + half, y + k);
+      s = clampi((s + 32) >> 6, 0, 255);
     } else {
-      fh[k] = c_chroma_taps4[fx * 4 + k];
-      fv[k] = c_chroma_taps4[fy * 4 + k];
+      for (int j = 0; j < ntap; j++) {
+        int t = 0;
+        for (int k = 0; k < ntap; k++) t += mc_tap(F.th0, F.th1, k) * at(x + k, y + j);
+        s += mc_tap(F.tv0, F.tv1, j) * (int16_t)t;
+      }
+      s = clampi((s + 2048) >> 12, 0, 255);
     }
-  }
-  const int wx0 = x0 + dx - half, wy0 = y0 + dy - half, ww = n + ntap - 1;
-  p_mc_sync();  // the window buffer is free
-  for (int i = tid; i < ww * ww; i += nth) {
-    const int yy = i / ww, xx = i % ww;
-    const int gx = clampi(wx0 + xx, 0, pw - 1), gy = clampi(wy0 + yy, 0, ph - 1);
-    S.win[yy][xx] = (int16_t)ref[(size_t)gy * rstride + gx];
-  }
-  p_mc_sync();
-  if (fx != 0 && fy != 0) {  // horizontal pass over every window row (shift1 is 0 at 8 bits)
-    for (int i = tid; i < n * ww; i += nth) {
-      const int x = i % n, yy = i / n;
-      int s = 0;
-      for (int k = 0; k < ntap; k++) s += fh[k] * S.win[yy][x + k];
-      S.tmp[yy][x] = (int16_t)s;
-    }
-    p_mc_sync();
-  }
-  for (int i = tid; i < n * n; i += nth) {
-    const int x = i % n, y = i / n;
-    int p;
-    if (fx == 0 && fy == 0) {
-      p = S.win[y + half][x + half];
-    } else if (fy == 0) {
-      int s = 0;
-      for (int k = 0; k < ntap; k++) s += fh[k] * S.win[y + half][x + k];
-      p = clampi((s + 32) >> 6, 0, 255);
-    } else if (fx == 0) {
-      int s = 0;
-      for (int k = 0; k < ntap; k++) s += fv[k] * S.win[y + k][x + half];
-      p = clampi((s + 32) >> 6, 0, 255);
-    } else {
-      int s = 0;
-      for (int k = 0; k < ntap; k++) s += fv[k] * S.tmp[y + k][x];
-      p = clampi((s + 2048) >> 12, 0, 255);
-    }
-    pred[i] = (int16_t)p;
+    o[y * tw + x] = (int16_t)s;
   }
 }
 
+// The inter prediction of one 16-row tile (luma 32x16, chroma 16x16) of a
+// coding unit by one warp, raster into `pred`. (bx, by): the tile's position in
+// the component's plane.
+template <bool kLuma>
+__device__ __forceinline__ void p_predict_tile(const PPicDev& P, const vvcg_inter_cu& rec, int cu, int comp, int bx,
+                                               int by, int16_t* pred, McWs& S, int lane) {
+  constexpr int tw = kLuma ? 32 : 16, ntap = kLuma ? 8 : 4, half = ntap / 2 - 1;
+  if (!((rec.inter_dir & 1) && rec.ref_idx[0] >= 0)) {  // predict_inter_pu without a usable list: 128
+    for (int i = lane; i < tw * 8; i += 32) reinterpret_cast<uint32_t*>(pred)[i] = 128u | 128u << 16;
+    return;
+  }
+  const McParams Pm = p_params<kLuma>(P, rec, comp);
+  const McFilter F = p_filter<kLuma>(Pm, rec);
+  if (!mc_tile<ntap, false>(Pm, F, bx + F.dx - half, by + F.dy - half, tw, 16, pred, tw, S, lane))
+    p_tile_wide<kLuma>(&P, &P.cus[cu], comp, bx, by, pred);
+}
+
 // Grid: (CTUs of the largest picture of the level, pictures of the level).
-// Warp 0 turns the luma levels into the residual while warps 1 and 2 do the
-// chroma ones and then, with warp 3, the three predictions; all four warps
-// then add, clip and store.
-__global__ void __launch_bounds__(kPWarps * 32, 7)
+// The unit's work is cut into near-equal parts: warp 0 turns the luma levels
+// into the residual, warps 1 and 2 a chroma component's and then predict half
+// of the luma, warp 3 predicts Cb and Cr; then all four add, clip and store.
+// Which warp is which rotates with the unit, because a warp's place decides
+// its scheduler: fixed, 298 us for eight 1920x1088 pictures; rotated, 265; with
+// sparse levels read straight into the transform tile, 218 (27 us a picture).
+// Before the 16-bit transforms and packed filters it took 644 us. What bounds it
+// now is instruction fetch and the wait for the slowest part.
+__global__ void __launch_bounds__(kPWarps * 32, 8)
 k_p_cu(const PPicDev* __restrict__ pics, const int16_t* __restrict__ levels, uint64_t n_levels, uint32_t* status) {
-  __shared__ __align__(16) int16_t ws_luma[tu_inv_ws(1024)];     // the luma warp's transform tiles
-  __shared__ __align__(16) int16_t ws_chroma[2][tu_inv_ws(256)];  // the chroma warps' tiles
-  __shared__ __align__(16) PMcSmem mc;
+  constexpr int kWs = sizeof(McWs) > tu_inv_ws(256) * 2 ? sizeof(McWs) : tu_inv_ws(256) * 2;
+  __shared__ __align__(16) int16_t ws_luma[tu_inv_ws(1024)];
+  __shared__ __align__(16) unsigned char ws[3][kWs];  // warps 1..3: transform tiles, then prediction window
   __shared__ __align__(16) int16_t res[1024 + 2 * 256];
   __shared__ __align__(16) int16_t pred[1024 + 2 * 256];
-  __shared__ __align__(16) int16_t dense[1024 + 2 * 256];  // sparse TBs expanded (same layout as res)
   const PPicDev& P = pics[blockIdx.y];
   const int cu = blockIdx.x;
   if (cu >= P.gw * P.gh) return;
   const vvcg_inter_cu rec = P.cus[cu];
   const int bx = (cu % P.gw) * 32, by = (cu / P.gw) * 32;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, wid = ((threadIdx.x >> 5) + cu) & 3;
   if (wid < 3) {
     const int c = wid, n = c ? 256 : 1024, off_res = c == 0 ? 0 : (c == 1 ? 1024 : 1280);
     int16_t* r = res + off_res;
     bool coded = (rec.cbf >> c) & 1;
     if (coded) {
       const int off = rec.level_off[c];
-      const int16_t* src = levels + off;
       bool ok = off >= 0 && !(rec.tu_tools >> 3);
+      int cnt = -1;
       if (ok && (P.flags & 2)) {  // sparse: count, unused word, (index, level) pairs
-        const int cnt = (off & 1) || (uint64_t)off + 2 > n_levels ? -1 : levels[off];
-        ok = cnt >= 0 && cnt <= n && (uint64_t)off + 2 + 2 * (uint64_t)cnt <= n_levels &&
-             expand_sparse(levels + off, cnt, n, dense + off_res, lane);
-        src = dense + off_res;
+        cnt = (off & 1) || (uint64_t)off + 2 > n_levels ? -1 : levels[off];
+        ok = cnt >= 0 && cnt <= n && (uint64_t)off + 2 + 2 * (uint64_t)cnt <= n_levels;
       } else if (ok) {
         ok = (uint64_t)off + (uint64_t)n <= n_levels;
       }
@@ -160,30 +150,57 @@ k_p_cu(const PPicDev* __restrict__ pics, const int16_t* __restrict__ levels, uin
         t.flags = ts ? VVCG_TU_TRANSFORM_SKIP : ((P.flags & 1) ? VVCG_TU_DEP_QUANT : 0);
         t.mts_idx = t.lfnst_idx = t.lfnst_mode = 0;
         t.in_off = t.out_off = 0;
-        warp_tu_inverse(t, src, r, c ? ws_chroma[c - 1] : ws_luma, lane);
+        if (!warp_tu_inverse(t, levels + off + (cnt >= 0 ? 2 : 0), r,
+                             c ? reinterpret_cast<int16_t*>(ws[c - 1]) : ws_luma, lane, 0, cnt) &&
+            lane == 0)
+          atomicOr(status, kStatusBadRecord);
       }
     }
     if (!coded)
-      for (int i = lane; i < n; i += 32) r[i] = 0;
+      for (int i = lane; i < n / 2; i += 32) reinterpret_cast<uint32_t*>(r)[i] = 0;
+    __syncwarp();
   }
-  if (wid >= 1)
-    for (int c = 0; c < 3; c++)
-      p_predict_component(P, rec, c, bx, by, pred + (c == 0 ? 0 : (c == 1 ? 1024 : 1280)), mc, threadIdx.x - 32);
+  if (wid >= 1) {
+    McWs& S = *reinterpret_cast<McWs*>(ws[wid - 1]);
+    if (wid < 3) {
+      p_predict_tile<true>(P, rec, cu, 0, bx, by + 16 * (wid - 1), pred + 512 * (wid - 1), S, lane);
+    } else {
+#pragma unroll 1
+      for (int c = 1; c <= 2; c++) {
+        p_predict_tile<false>(P, rec, cu, c, bx / 2, by / 2, pred + 768 + 256 * c, S, lane);
+        __syncwarp();
+      }
+    }
+  }
   __syncthreads();
-  // reconstruction: clip(prediction + residual), two samples per store
-  for (int i = threadIdx.x; i < (1024 + 512) / 2; i += blockDim.x) {
-    const int e = 2 * i;
-    const int comp = e < 1024 ? 0 : (e < 1280 ? 1 : 2);
-    const int n = comp ? 16 : 32, base = comp == 0 ? 0 : (comp == 1 ? 1024 : 1280);
-    const int k = e - base, x = k % n, y = k / n;
-    const int x0 = comp ? bx / 2 : bx, y0 = comp ? by / 2 : by;
-    const uint32_t pv = *reinterpret_cast<const uint32_t*>(&pred[e]);
-    const uint32_t rv = *reinterpret_cast<const uint32_t*>(&res[e]);
-    const int v0 = clampi((int)(int16_t)(pv & 0xFFFFu) + (int)(int16_t)(rv & 0xFFFFu), 0, 255);
-    const int v1 = clampi((int)(int16_t)(pv >> 16) + (int)(int16_t)(rv >> 16), 0, 255);
-    *reinterpret_cast<uint32_t*>(P.out[comp] + (size_t)(y0 + y) * P.stride[comp] + x0 + x) =
-        (uint32_t)v0 | ((uint32_t)v1 << 16);
+  // reconstruction: clip(prediction + residual), eight samples a step
+  for (int r = threadIdx.x; r < (1024 + 512) / 8; r += blockDim.x) {
+    const int comp = r < 128 ? 0 : (r < 160 ? 1 : 2);
+    const int k = comp == 0 ? r : (comp == 1 ? r - 128 : r - 160);
+    const int x = comp ? 8 * (k & 1) : 8 * (k & 3), y = comp ? k >> 1 : k >> 2;
+    const uint4 p = *reinterpret_cast<const uint4*>(&pred[8 * r]), d = *reinterpret_cast<const uint4*>(&res[8 * r]);
+    constexpr uint32_t top = 0x00FF00FFu;
+    *reinterpret_cast<uint4*>(P.out[comp] + (size_t)((comp ? by / 2 : by) + y) * P.stride[comp] + (comp ? bx / 2 : bx) +
+                              x) = make_uint4(add_clip2(p.x, d.x, top), add_clip2(p.y, d.y, top),
+                                              add_clip2(p.z, d.z, top), add_clip2(p.w, d.w, top));
   }
+}
+
+// The CTU-boundary deblocking's cells: each CTU's own L0 motion and cbfs
+// (slice.rs:2319-2326, :2438-2444), one thread per record.
+__global__ void k_p_cells(const vvcg_inter_cu* __restrict__ cus, uint32_t n, vvcg_ctu_motion* __restrict__ cells) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const vvcg_inter_cu& r = cus[i];
+  vvcg_ctu_motion m;
+  for (int j = 0; j < 3; j++) {
+    m.mv[j][0] = r.mv[0][0];
+    m.mv[j][1] = r.mv[0][1];
+    m.ref[j] = r.ref_idx[0];
+    m.reserved[j] = 0;
+  }
+  m.cbf = r.cbf & 7;
+  cells[i] = m;
 }
 
 }  // namespace vvcg
@@ -345,7 +362,7 @@ extern "C" vvcg_status vvcg_decode_p_batch(vvcg_ctx* ctx, const vvcg_p_pic* pics
   const uint64_t ncu = (uint64_t)num_cus;
   CK(s.d_cus.reserve(ncu * sizeof(vvcg_inter_cu)), "cudaMalloc");
   CK(s.d_levels.reserve(std::max<uint64_t>(num_levels, 1) * sizeof(int16_t)), "cudaMalloc");
-  CK(s.d_cells.reserve((uint64_t)num_pics * gw * gh * sizeof(vvcg_ctu_motion)), "cudaMalloc");
+  CK(s.d_cells.reserve(ncu * sizeof(vvcg_ctu_motion)), "cudaMalloc");
   CK(s.d_pics.reserve(num_pics * sizeof(vvcg::PPicDev)), "cudaMalloc");
   CK(s.d_status.reserve(sizeof(uint32_t)), "cudaMalloc");
   CK(cudaMemcpyAsync(s.d_cus.p, cus, ncu * sizeof(vvcg_inter_cu), cudaMemcpyHostToDevice, ctx->stream), "upload");
@@ -353,7 +370,6 @@ extern "C" vvcg_status vvcg_decode_p_batch(vvcg_ctx* ctx, const vvcg_p_pic* pics
     CK(cudaMemcpyAsync(s.d_levels.p, levels, num_levels * sizeof(int16_t), cudaMemcpyHostToDevice, ctx->stream),
        "upload");
   CK(cudaMemsetAsync(s.d_status.p, 0, sizeof(uint32_t), ctx->stream), "memset");
-  std::vector<vvcg_ctu_motion> cells((size_t)num_pics * gw * gh);
   std::vector<std::vector<vvcg::PPicDev>> by_level(num_levels_dep);
   for (uint32_t i = 0; i < num_pics; i++) {
     const vvcg_p_pic& p = pics[i];
@@ -374,22 +390,7 @@ extern "C" vvcg_status vvcg_decode_p_batch(vvcg_ctx* ctx, const vvcg_p_pic* pics
     d.num_refs = p.num_refs;
     d.flags = ((p.options & VVCG_SLICE_DEP_QUANT) ? 1u : 0u) | (p.sparse ? 2u : 0u);
     by_level[level[i]].push_back(d);
-    // slice.rs:2319-2326 / :2438-2444: each CTU's own L0 motion and cbfs
-    for (uint32_t k = 0; k < gw * gh; k++) {
-      const vvcg_inter_cu& r = cus[p.cu_offset + k];
-      vvcg_ctu_motion& m = cells[(size_t)i * gw * gh + k];
-      memset(&m, 0, sizeof(m));
-      for (int j = 0; j < 3; j++) {
-        m.mv[j][0] = r.mv[0][0];
-        m.mv[j][1] = r.mv[0][1];
-        m.ref[j] = r.ref_idx[0];
-      }
-      m.cbf = r.cbf & 7;
-    }
   }
-  CK(cudaMemcpyAsync(s.d_cells.p, cells.data(), cells.size() * sizeof(vvcg_ctu_motion), cudaMemcpyHostToDevice,
-                     ctx->stream),
-     "upload");
   std::vector<vvcg::PPicDev> flat;
   std::vector<size_t> start;
   for (auto& L : by_level) {
@@ -399,18 +400,56 @@ extern "C" vvcg_status vvcg_decode_p_batch(vvcg_ctx* ctx, const vvcg_p_pic* pics
   CK(cudaMemcpyAsync(s.d_pics.p, flat.data(), flat.size() * sizeof(vvcg::PPicDev), cudaMemcpyHostToDevice,
                      ctx->stream),
      "upload");
+  // deblocking passes of the pictures that enable it, level by level: luma V,
+  // chroma V, luma H, chroma H; the cells of all records
+  std::vector<DbfPass>& passes = ctx->dbf_ctu;
+  passes.clear();
+  struct LevelPasses {
+    size_t at[4];
+    uint32_t pics;
+  };
+  std::vector<LevelPasses> dbf(num_levels_dep, LevelPasses{{0, 0, 0, 0}, 0});
+  for (int L = 0; L < num_levels_dep; L++) {
+    std::vector<DbfPass> kind[4];
+    for (uint32_t i = 0; i < num_pics; i++) {
+      if (level[i] != L || !(pics[i].options & VVCG_SLICE_DEBLOCK)) continue;
+      uint16_t* planes[3] = {s.plane((uint32_t)pics[i].out_slot, 0), s.plane((uint32_t)pics[i].out_slot, 1),
+                             s.plane((uint32_t)pics[i].out_slot, 2)};
+      DbfPass six[6];
+      ctu_edge_passes(planes, s.stride, s.w, s.h, 32, pics[i].qp,
+                      (const vvcg_ctu_motion*)s.d_cells.p + pics[i].cu_offset, six);
+      kind[0].push_back(six[0]);
+      kind[1].insert(kind[1].end(), six + 1, six + 3);
+      kind[2].push_back(six[3]);
+      kind[3].insert(kind[3].end(), six + 4, six + 6);
+      dbf[L].pics++;
+    }
+    for (int k = 0; k < 4; k++) {
+      dbf[L].at[k] = passes.size();
+      passes.insert(passes.end(), kind[k].begin(), kind[k].end());
+    }
+  }
+  if (!passes.empty()) {
+    CK(ctx->d_dbf_ctu.reserve(sizeof(DbfPass) * passes.size()), "cudaMalloc");
+    CK(cudaMemcpyAsync(ctx->d_dbf_ctu.p, passes.data(), sizeof(DbfPass) * passes.size(), cudaMemcpyHostToDevice,
+                       ctx->stream),
+       "upload");
+    vvcg::k_p_cells<<<(num_cus + 255) / 256, 256, 0, ctx->stream>>>((const vvcg_inter_cu*)s.d_cus.p, num_cus,
+                                                                     (vvcg_ctu_motion*)s.d_cells.p);
+    CK(cudaGetLastError(), "cells launch");
+    ctx->launches++;
+  }
   const vvcg::PPicDev* dp = (const vvcg::PPicDev*)s.d_pics.p;
   for (int L = 0; L < num_levels_dep; L++) {
     vvcg::k_p_cu<<<dim3(gw * gh, (unsigned)by_level[L].size()), vvcg::kPWarps * 32, 0, ctx->stream>>>(
         dp + start[L], (const int16_t*)s.d_levels.p, num_levels, (uint32_t*)s.d_status.p);
     ctx->launches++;
     CK(cudaGetLastError(), "P-picture launch");
-    for (uint32_t i = 0; i < num_pics; i++) {
-      if (level[i] != L || !(pics[i].options & VVCG_SLICE_DEBLOCK)) continue;
-      uint16_t* planes[3] = {s.plane((uint32_t)pics[i].out_slot, 0), s.plane((uint32_t)pics[i].out_slot, 1),
-                             s.plane((uint32_t)pics[i].out_slot, 2)};
-      vvcg_status st = vvcg_deblock_ctu_edges_dev(ctx, planes, s.stride, s.w, s.h, 32, pics[i].qp,
-                                                  (const vvcg_ctu_motion*)s.d_cells.p + (size_t)i * gw * gh);
+    if (dbf[L].pics) {
+      const DbfPass* d = (const DbfPass*)ctx->d_dbf_ctu.p;
+      const vvcg_status st = launch_ctu_edges(ctx, d + dbf[L].at[0], d + dbf[L].at[1], d + dbf[L].at[2],
+                                              d + dbf[L].at[3], &passes[dbf[L].at[0]], &passes[dbf[L].at[1]],
+                                              &passes[dbf[L].at[2]], &passes[dbf[L].at[3]], dbf[L].pics);
       if (st != VVCG_OK) return st;
     }
   }

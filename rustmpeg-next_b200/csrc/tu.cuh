@@ -462,7 +462,7 @@ __device__ __forceinline__ int dq_step(int st, int level) {
 
 // predict.rs:4224-4240: saturating running sums along rows or down columns,
 // one lane a line, in place.
-__device__ __forceinline__ void tu_bdpcm(int16_t* p, int stride, const TuShape& S, bool vert, int lane) {
+__device__ __noinline__ void tu_bdpcm(int16_t* p, int stride, const TuShape& S, bool vert, int lane) {
   const int lines = vert ? S.w : S.h, len = vert ? S.h : S.w;
   const int step = vert ? stride : 1, lstep = vert ? 1 : stride;
   for (int l = lane; l < lines; l += 32) {
@@ -481,29 +481,62 @@ __device__ __forceinline__ void tu_bdpcm(int16_t* p, int stride, const TuShape& 
 // the BDPCM of :4055-4060). The residual goes to `out` with row stride
 // `ostride` (0: the unit's width). ws: tu_inv_ws int16 entries, 16-byte
 // aligned. Rows and columns past the last nonzero coefficient hold zeros and
-// are left out of the sums.
-__device__ void warp_tu_inverse(const vvcg_tu_rec& r, const int16_t* __restrict__ in,
-                                int16_t* __restrict__ out, int16_t* ws, int lane, int ostride = 0) {
+// are left out of the sums. The levels are raster, or with npairs >= 0 the
+// sparse form: `in` holds npairs (raster index, level) pairs, 4-byte aligned,
+// with rising indices (units of at most 32x32); false when an index is outside
+// the unit or not above the one before it (that entry is left out).
+__device__ bool warp_tu_inverse(const vvcg_tu_rec& r, const int16_t* __restrict__ in,
+                                int16_t* __restrict__ out, int16_t* ws, int lane, int ostride = 0, int npairs = -1) {
   TuShape S;
   tu_shape(r, S);
   const int bd = r.bit_depth, qp = r.qp;
   const int os = ostride ? ostride : S.w;
-  const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0 && S.n >= 256;  // 8 levels a lane and load
+  const bool sparse = npairs >= 0;
+  const bool vec = !sparse && (reinterpret_cast<uintptr_t>(in) & 15) == 0 && S.n >= 256;  // 8 levels a lane and load
+  bool ok = true;
+  // calls put(index, level) for this lane's sparse entries, each index checked
+  // against the entry before it, so that no two land on one coefficient
+  auto for_pairs = [&](auto&& put) {
+    const uint32_t* pr = reinterpret_cast<const uint32_t*>(in);
+    int prev_last = -1;
+    for (int base = 0; base < npairs; base += 32) {
+      const int i = base + lane;
+      const bool have = i < npairs;
+      const uint32_t e = have ? pr[i] : (uint32_t)S.n;
+      const int pos = (int)(e & 0xFFFFu), L = (int)(int16_t)(e >> 16);
+      int prev = __shfl_up_sync(0xffffffffu, pos, 1);
+      if (lane == 0) prev = prev_last;
+      if (have) {
+        if (pos >= S.n || pos <= prev)
+          ok = false;
+        else if (L != 0)
+          put(pos, L);
+      }
+      prev_last = __shfl_sync(0xffffffffu, pos, 31);
+    }
+    ok = __all_sync(0xffffffffu, ok);
+  };
   const bool bdpcm = (r.flags & (VVCG_TU_BDPCM_HOR | VVCG_TU_BDPCM_VER)) != 0;
   if (r.flags & VVCG_TU_TRANSFORM_SKIP) {
     // BDPCM sums in the workspace, except for 64x64, which does not fit
     const bool tile = bdpcm && S.n < 4096;
     int16_t* d = tile ? ws : out;
     const int ds = tile ? S.w + 2 : os;
-    for (int i = lane; i < S.n; i += 32)
-      d[(size_t)(i >> S.lw) * ds + (i & (S.w - 1))] = (int16_t)tu_dequant_ts(in[i], qp);
+    if (sparse) {
+      for (int i = lane; i < S.n; i += 32) d[(size_t)(i >> S.lw) * ds + (i & (S.w - 1))] = 0;
+      __syncwarp();
+      for_pairs([&](int i, int L) { d[(size_t)(i >> S.lw) * ds + (i & (S.w - 1))] = (int16_t)tu_dequant_ts(L, qp); });
+    } else {
+      for (int i = lane; i < S.n; i += 32)
+        d[(size_t)(i >> S.lw) * ds + (i & (S.w - 1))] = (int16_t)tu_dequant_ts(in[i], qp);
+    }
     __syncwarp();
     if (bdpcm) tu_bdpcm(d, ds, S, (r.flags & VVCG_TU_BDPCM_VER) != 0, lane);
     if (tile)
       for (int i = lane; i < S.n; i += 32)
         out[(size_t)(i >> S.lw) * os + (i & (S.w - 1))] = ws[(i >> S.lw) * ds + (i & (S.w - 1))];
     __syncwarp();
-    return;
+    return ok;
   }
   // coefficients transposed: C[x][y], x < 32, y < 32
   const int tw = min(S.w, 32), th = min(S.h, 32);
@@ -541,7 +574,9 @@ __device__ void warp_tu_inverse(const vvcg_tu_rec& r, const int16_t* __restrict_
     }
     C[x * pc + y] = (int16_t)v;
   };
-  if (vec) {
+  if (sparse) {
+    for_pairs(put);
+  } else if (vec) {
     for (int v0 = 0; v0 < S.n; v0 += 1024) {
 #pragma unroll
       for (int v = 0; v < 4; v++) {
@@ -642,13 +677,13 @@ __device__ void warp_tu_inverse(const vvcg_tu_rec& r, const int16_t* __restrict_
     }
     __syncwarp();
     if (bdpcm) tu_bdpcm(out, os, S, (r.flags & VVCG_TU_BDPCM_VER) != 0, lane);
-    return;
+    return ok;
   }
   const int nc = min(S.w - S.sw, maxc + 1), nr = min(S.h - S.sh, maxr + 1);
   if (nc <= 0 || nr <= 0) {
     for (int i = lane; i < S.n; i += 32) out[(size_t)(i >> S.lw) * os + (i & (S.w - 1))] = 0;
     __syncwarp();
-    return;
+    return ok;
   }
   // coefficients the zero-out drops inside the last group (the other rows
   // and columns up to the groups read are zero already or not read)
@@ -664,6 +699,7 @@ __device__ void warp_tu_inverse(const vvcg_tu_rec& r, const int16_t* __restrict_
             TuStore{out, 1, os}, 1 << (19 - bd), 20 - bd, lane);
   __syncwarp();
   if (bdpcm) tu_bdpcm(out, os, S, (r.flags & VVCG_TU_BDPCM_VER) != 0, lane);
+  return ok;
 }
 
 // One warp: residual -> levels of one unit (slice.rs:690-760, level side).
@@ -893,38 +929,10 @@ constexpr int kResToolWarps = 4;
 // Records outside the ranges of vvcg_cu_rec.tu_tools, or with levels past the
 // pool, set the bad-record status and are skipped.
 // Grid: (ceil(max CUs per picture / kResToolWarps), pictures).
-// A sparse TB's (raster index, level) pairs expanded into n dense levels;
-// false when an index is outside the TB or not above the one before it.
-__device__ bool expand_sparse(const int16_t* __restrict__ lv, int count, int n, int16_t* dense, int lane) {
-  for (int i = lane; i < n; i += 32) dense[i] = 0;
-  __syncwarp();
-  const uint32_t* pr = reinterpret_cast<const uint32_t*>(lv + 2);
-  bool ok = true;
-  int prev_last = -1;
-  for (int base = 0; base < count; base += 32) {
-    const int i = base + lane;
-    const bool have = i < count;
-    const uint32_t e = have ? pr[i] : (uint32_t)n;
-    const int pos = (int)(e & 0xFFFFu);
-    int prev = __shfl_up_sync(0xffffffffu, pos, 1);
-    if (lane == 0) prev = prev_last;
-    if (have) {
-      if (pos >= n || pos <= prev)
-        ok = false;
-      else
-        dense[pos] = (int16_t)(e >> 16);
-    }
-    prev_last = __shfl_sync(0xffffffffu, pos, 31);
-  }
-  __syncwarp();
-  return __all_sync(0xffffffffu, ok);
-}
-
 __global__ void __launch_bounds__(kResToolWarps * 32)
 k_residual_tools(const DevPic* __restrict__ pics, const int16_t* __restrict__ levels, uint64_t n_levels,
                  uint32_t* status) {
   __shared__ __align__(16) int16_t ws[kResToolWarps][tu_inv_ws(1024)];
-  __shared__ __align__(16) int16_t dense[kResToolWarps][1024];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const DevPic& P = pics[blockIdx.y];
   if (!(P.tools & VVCG_TOOL_TU_TOOLS)) return;
@@ -942,16 +950,15 @@ k_residual_tools(const DevPic* __restrict__ pics, const int16_t* __restrict__ le
     const int off = rec.level_off[c];
     if (off < 0) continue;
     const int w = c ? P.tb_cw : P.tb, h = c ? P.tb_ch : P.tb;
-    const int16_t* src = levels + off;
+    int cnt = -1;
+    bool ok = !bad_tools;
     if (sparse) {  // count at levels[off], pairs from off + 2 (off even)
-      const int cnt = (off & 1) || (uint64_t)off + 2 > n_levels ? -1 : levels[off];
-      if (bad_tools || cnt < 0 || cnt > w * h || (uint64_t)off + 2 + 2 * (uint64_t)cnt > n_levels ||
-          !expand_sparse(levels + off, cnt, w * h, dense[wid], lane)) {
-        if (lane == 0) atomicOr(status, kStatusBadRecord);
-        continue;
-      }
-      src = dense[wid];
-    } else if (bad_tools || (uint64_t)off + (uint64_t)(w * h) > n_levels) {
+      cnt = (off & 1) || (uint64_t)off + 2 > n_levels ? -1 : levels[off];
+      ok = ok && cnt >= 0 && cnt <= w * h && (uint64_t)off + 2 + 2 * (uint64_t)cnt <= n_levels;
+    } else {
+      ok = ok && (uint64_t)off + (uint64_t)(w * h) <= n_levels;
+    }
+    if (!ok) {
       if (lane == 0) atomicOr(status, kStatusBadRecord);
       continue;
     }
@@ -969,7 +976,8 @@ k_residual_tools(const DevPic* __restrict__ pics, const int16_t* __restrict__ le
     r.in_off = r.out_off = 0;
     const int x0 = c ? gx * P.tb / P.sub_w : gx * P.tb, y0 = c ? gy * P.tb / P.sub_h : gy * P.tb;
     int16_t* out = reinterpret_cast<int16_t*>(P.scratch[c]) + (size_t)y0 * P.stride[c] + x0;
-    warp_tu_inverse(r, src, out, ws[wid], lane, P.stride[c]);
+    if (!warp_tu_inverse(r, levels + off + (sparse ? 2 : 0), out, ws[wid], lane, P.stride[c], cnt) && lane == 0)
+      atomicOr(status, kStatusBadRecord);
   }
 }
 

@@ -2182,6 +2182,51 @@ extern "C" vvcg_status vvcg_gpm_blend_dev(vvcg_ctx* ctx, const vvcg_gpm_req* req
 // ---------------------------------------------------------------------------
 static_assert(sizeof(vvcg_ctu_motion) == 40, "CTU motion layout");
 
+namespace {
+
+// The six passes of one picture: luma V, Cb V, Cr V, luma H, Cb H, Cr H
+// (slice.rs:2305-2311: SliceQpY, derived_chroma_qp, lengths of min(ctu, 32) luma
+// and ctu/2 chroma transform sides).
+void ctu_edge_passes(uint16_t* const planes[3], const uint32_t stride[3], uint32_t width, uint32_t height, uint32_t ctu,
+                     uint8_t qp, const vvcg_ctu_motion* cells, DbfPass out[6]) {
+  const int w = (int)width, h = (int)height, cw = w / 2, ch = h / 2, c = (int)ctu, cc = c / 2;
+  const int cqp = std::min(63, std::max(0, (int)qp <= 26 ? (int)qp : (int)qp - 1));
+  const int lml = std::min(c, 32) >= 32 ? 7 : 3;
+  const int cols = w / c, rows = h / c;
+  out[0] = DbfPass{planes[0], (int32_t)stride[0], w, h, 8, c, c, (int)qp, 0, 0, 0, lml, lml, 1, cols - 1, h / 4,
+                   cells, cols, 0, c};
+  out[3] = DbfPass{planes[0], (int32_t)stride[0], w, h, 8, c, c, (int)qp, 0, 0, 0, lml, lml, 1, rows - 1, w / 4,
+                   cells, cols, 0, c};
+  for (int k = 1; k <= 2; k++) {
+    out[k] = DbfPass{planes[k], (int32_t)stride[k], cw, ch, 8, cc, cc, cqp, 0, 0, 0, 3, 3, 2, cols - 1, ch / 2,
+                     cells, cols, k, cc};
+    out[3 + k] = DbfPass{planes[k], (int32_t)stride[k], cw, ch, 8, cc, cc, cqp, 0, 0, 0, 3, 3, 2, rows - 1, cw / 2,
+                         cells, cols, k, cc};
+  }
+}
+
+// Launches the passes of `pics` pictures of one size (device arrays d*, host
+// copies of their first entries h*): vertical edges, then horizontal ones.
+vvcg_status launch_ctu_edges(vvcg_ctx* ctx, const DbfPass* dlv, const DbfPass* dcv, const DbfPass* dlh,
+                             const DbfPass* dch, const DbfPass* hlv, const DbfPass* hcv, const DbfPass* hlh,
+                             const DbfPass* hch, uint32_t pics) {
+  auto blocks = [](const DbfPass* p) { return (unsigned)((std::max(0, p->n_edges * p->n_segs) + 127) / 128); };
+  if (hlv->n_edges > 0) {
+    k_deblock_luma<true><<<dim3(blocks(hlv), pics), 128, 0, ctx->stream>>>(dlv, (int)pics);
+    k_deblock_chroma<true><<<dim3(blocks(hcv), 2 * pics), 128, 0, ctx->stream>>>(dcv, 2 * (int)pics);
+    ctx->launches += 2;
+  }
+  if (hlh->n_edges > 0) {
+    k_deblock_luma<false><<<dim3(blocks(hlh), pics), 128, 0, ctx->stream>>>(dlh, (int)pics);
+    k_deblock_chroma<false><<<dim3(blocks(hch), 2 * pics), 128, 0, ctx->stream>>>(dch, 2 * (int)pics);
+    ctx->launches += 2;
+  }
+  CK(cudaGetLastError(), "deblock launch");
+  return VVCG_OK;
+}
+
+}  // namespace
+
 extern "C" vvcg_status vvcg_deblock_ctu_edges_dev(vvcg_ctx* ctx, uint16_t* const planes[3], const uint32_t stride[3],
                                                   uint32_t width, uint32_t height, uint32_t ctu, uint8_t qp,
                                                   const vvcg_ctu_motion* cells) {
@@ -2192,48 +2237,20 @@ extern "C" vvcg_status vvcg_deblock_ctu_edges_dev(vvcg_ctx* ctx, uint16_t* const
     return fail(ctx, VVCG_INVALID_INPUT, "picture size must be a nonzero multiple of the CTU size");
   if ((uint64_t)width * height > kMaxLumaSamples) return fail(ctx, VVCG_LIMIT_EXCEEDED, "picture too large");
   if (qp > 63) return fail(ctx, VVCG_INVALID_INPUT, "QP above 63");
-  const int w = (int)width, h = (int)height, cw = w / 2, ch = h / 2, c = (int)ctu, cc = c / 2;
   for (int k = 0; k < 3; k++)
-    if (!planes[k] || stride[k] < (uint32_t)(k ? cw : w) || (stride[k] & 7) ||
+    if (!planes[k] || stride[k] < (k ? width / 2 : width) || (stride[k] & 7) ||
         (reinterpret_cast<uintptr_t>(planes[k]) & 15))
       return fail(ctx, VVCG_INVALID_INPUT,
                   "plane %d: needs a 16-byte aligned pointer and a stride >= the width that is a multiple of 8", k);
   CK(cudaSetDevice(ctx->device), "cudaSetDevice");
-  // slice.rs:2305-2311: SliceQpY, derived_chroma_qp, lengths of min(ctu, 32)
-  // luma and ctu/2 chroma transform sides
-  const int cqp = std::min(63, std::max(0, (int)qp <= 26 ? (int)qp : (int)qp - 1));
-  const int lml = std::min(c, 32) >= 32 ? 7 : 3;
-  const int cols = w / c, rows = h / c;
   auto& v = ctx->dbf_ctu;
-  v.clear();
-  // luma V, Cb V, Cr V, luma H, Cb H, Cr H
-  v.push_back(DbfPass{planes[0], (int32_t)stride[0], w, h, 8, c, c, (int)qp, 0, 0, 0, lml, lml, 1, cols - 1, h / 4,
-                      cells, cols, 0, c});
-  for (int k = 1; k <= 2; k++)
-    v.push_back(DbfPass{planes[k], (int32_t)stride[k], cw, ch, 8, cc, cc, cqp, 0, 0, 0, 3, 3, 2, cols - 1, ch / 2,
-                        cells, cols, k, cc});
-  v.push_back(DbfPass{planes[0], (int32_t)stride[0], w, h, 8, c, c, (int)qp, 0, 0, 0, lml, lml, 1, rows - 1, w / 4,
-                      cells, cols, 0, c});
-  for (int k = 1; k <= 2; k++)
-    v.push_back(DbfPass{planes[k], (int32_t)stride[k], cw, ch, 8, cc, cc, cqp, 0, 0, 0, 3, 3, 2, rows - 1, cw / 2,
-                        cells, cols, k, cc});
+  v.resize(6);
+  ctu_edge_passes(planes, stride, width, height, ctu, qp, cells, v.data());
   CK(ctx->d_dbf_ctu.reserve(sizeof(DbfPass) * v.size()), "cudaMalloc");
   CK(cudaMemcpyAsync(ctx->d_dbf_ctu.p, v.data(), sizeof(DbfPass) * v.size(), cudaMemcpyHostToDevice, ctx->stream),
      "upload");
   const DbfPass* d = (const DbfPass*)ctx->d_dbf_ctu.p;
-  auto blocks = [](const DbfPass& p) { return (unsigned)((std::max(0, p.n_edges * p.n_segs) + 127) / 128); };
-  if (cols > 1) {
-    k_deblock_luma<true><<<dim3(blocks(v[0]), 1), 128, 0, ctx->stream>>>(d, 1);
-    k_deblock_chroma<true><<<dim3(blocks(v[1]), 2), 128, 0, ctx->stream>>>(d + 1, 2);
-    ctx->launches += 2;
-  }
-  if (rows > 1) {
-    k_deblock_luma<false><<<dim3(blocks(v[3]), 1), 128, 0, ctx->stream>>>(d + 3, 1);
-    k_deblock_chroma<false><<<dim3(blocks(v[4]), 2), 128, 0, ctx->stream>>>(d + 4, 2);
-    ctx->launches += 2;
-  }
-  CK(cudaGetLastError(), "deblock launch");
-  return VVCG_OK;
+  return launch_ctu_edges(ctx, d, d + 1, d + 3, d + 4, &v[0], &v[1], &v[3], &v[4], 1);
 }
 
 // ---------------------------------------------------------------------------
