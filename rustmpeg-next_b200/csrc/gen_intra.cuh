@@ -1,5 +1,5 @@
 // Intra prediction of the general decoding path (crates/rustmpeg-video/src/
-// vvc/decode_general.rs), one warp per transform block: reference samples
+// vvc/decode_general.rs), a group of whole warps per transform block: reference samples
 // with the decoded-map availability and nearest-available substitution of
 // Gen::gather_len (:4260-4341) and Gen::gather_mrl (:4542-4632), the ISP
 // reference lengths of isp_refs (:4634-4648), predict_luma (:4650-4732),
@@ -8,8 +8,7 @@
 // :4001-4024). The predictors are those of predict.rs (planar :1688, DC
 // :1722, PDPC :1739, predict_angular_with_params_bd :1776-1958, BDPCM :1993).
 #pragma once
-#include "vvcg_device.cuh"
-#include "vvcg_tables_dev.cuh"
+#include "intra_group.cuh"
 
 namespace vvcg {
 
@@ -29,7 +28,7 @@ struct GiWs {
   int16_t above[kGiRef], left[kGiRef];  // gathered references (gather_len)
   int16_t rowa[kGiRef], rowl[kGiRef];   // MrlRefSamples rows
   int16_t ba[kGiRef], bl[kGiRef];       // base refs for planar / DC (filtered or not)
-  int tl, btl, nrowa, nrowl, off;
+  int tl, btl, nrowa, nrowl, off, ft, fl;
 };
 
 struct GiAng {
@@ -89,103 +88,139 @@ __device__ __forceinline__ bool gi_decoded(const vvcg_gen_intra_state& S, bool l
   if (x < 0 || y < 0) return false;
   if (luma) {
     if (x >= (int)S.width || y >= (int)S.height) return false;
-    return S.dec_y[(size_t)(y >> 2) * (S.width >> 2) + (x >> 2)] != 0;
+    return __ldcg(S.dec_y + (size_t)(y >> 2) * (S.width >> 2) + (x >> 2)) != 0;
   }
   if (x >= (int)(S.width >> 1) || y >= (int)(S.height >> 1)) return false;
-  return S.dec_c[(size_t)y * (S.width >> 1) + x] != 0;
+  return __ldcg(S.dec_c + (size_t)y * (S.width >> 1) + x) != 0;
 }
 
+// Samples and decoded maps are read from L2: other CTAs of the launch write them.
 __device__ __forceinline__ int gi_get(const vvcg_gen_intra_state& S, int c, int x, int y) {
-  return S.plane[c][(size_t)y * S.stride[c] + x];
+  return __ldcg(S.plane[c] + (size_t)y * S.stride[c] + x);
 }
 
-// One side of Gen::gather_len / gather_mrl: dst[k] (k < len) = the sample at
-// position k when available, else the nearest available one before it, else
-// `fb` (the other fallbacks, resolved by the caller). `av` / `pos` give a
-// position's availability and plane coordinates. Returns the first available
-// sample (or -1) through *first.
+// One side of Gen::gather_len / gather_mrl by one warp: dst[k] (k < len) = the
+// sample at position k when available, else the nearest available one before
+// it, else -1 (the other fallbacks are the caller's). `av` / `pos` give a
+// position's availability and plane coordinates. The first available sample
+// (or -1) goes to *first. load() issues a chunk pair's loads (sample and
+// availability together, one memory round trip), put() uses them.
+struct GiSide {
+  int v[2];
+  bool a[2];
+};
 template <class Avail, class Pos>
-__device__ void gi_fill_side(const vvcg_gen_intra_state& S, int c, int len, int16_t* dst, Avail av, Pos pos,
-                             int* first_val) {
+__device__ __forceinline__ GiSide gi_side_load(const vvcg_gen_intra_state& S, int c, int k0, int len, Avail av,
+                                               Pos pos) {
   const int lane = threadIdx.x & 31;
-  int carry = -1;  // value of the last available position of earlier chunks
-  int first = -1;
   const int pw = c ? (int)S.width >> 1 : (int)S.width, ph = c ? (int)S.height >> 1 : (int)S.height;
-  for (int k0 = 0; k0 < len; k0 += 32) {
-    const int k = k0 + lane;
-    // the sample is loaded with the availability lookup, not after it (one
-    // memory round trip instead of two); unavailable ones are dropped
+  GiSide r;
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const int k = k0 + 32 * q + lane;
     int px = 0, py = 0;
     if (k < len) pos(k, &px, &py);
     const bool inplane = k < len && px >= 0 && py >= 0 && px < pw && py < ph;
-    int v = inplane ? gi_get(S, c, px, py) : -1;
-    const bool a = k < len && av(k);
-    if (!a) v = -1;
-    const uint32_t m = __ballot_sync(0xFFFFFFFFu, a);
+    r.v[q] = inplane ? gi_get(S, c, px, py) : -1;
+    r.a[q] = k < len && av(k);
+  }
+  return r;
+}
+__device__ __forceinline__ void gi_side_put(const GiSide& r, int k0, int len, int16_t* dst, int& carry, int& first) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const int k = k0 + 32 * q + lane;
+    const int v = r.a[q] ? r.v[q] : -1;
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, r.a[q]);
     if (first < 0 && m) first = __shfl_sync(0xFFFFFFFFu, v, __ffs(m) - 1);
     const uint32_t below = m & ((1u << lane) - 1u);
     const int src = below ? 31 - __clz(below) : -1;
     const int pv = __shfl_sync(0xFFFFFFFFu, v, src < 0 ? 0 : src);
-    if (k < len) dst[k] = (int16_t)(a ? v : (src >= 0 ? pv : carry));
+    if (k < len) dst[k] = (int16_t)(r.a[q] ? v : (src >= 0 ? pv : carry));
     if (m) carry = __shfl_sync(0xFFFFFFFFu, v, 31 - __clz(m));
   }
-  *first_val = first;
-  __syncwarp();
+}
+
+// Both sides of a block's references (comp c) into W.above / W.left with their
+// first available samples in W.ft / W.fl; av* / pos* as for one side. The
+// group's first warp takes the row above and its last the column left (one
+// warp: both, all loads of 64 positions a side before their first use).
+template <class AvA, class PosA, class AvL, class PosL>
+__device__ __forceinline__ void gi_fill(const Grp& g, const vvcg_gen_intra_state& S, int c, int top_len, int left_len,
+                                        GiWs& W, AvA ava, PosA posa, AvL avl, PosL posl) {
+  const bool top = g.tid < 32, left = g.tid >= g.n - 32;
+  GiSide a, l;
+  if (top) a = gi_side_load(S, c, 0, top_len, ava, posa);
+  if (left) l = gi_side_load(S, c, 0, left_len, avl, posl);
+  if (top) {
+    int carry = -1, first = -1;
+    gi_side_put(a, 0, top_len, W.above, carry, first);
+    for (int k0 = 64; k0 < top_len; k0 += 64)
+      gi_side_put(gi_side_load(S, c, k0, top_len, ava, posa), k0, top_len, W.above, carry, first);
+    if (g.tid == 0) W.ft = first;
+  }
+  if (left) {
+    int carry = -1, first = -1;
+    gi_side_put(l, 0, left_len, W.left, carry, first);
+    for (int k0 = 64; k0 < left_len; k0 += 64)
+      gi_side_put(gi_side_load(S, c, k0, left_len, avl, posl), k0, left_len, W.left, carry, first);
+    if (g.tid == g.n - 1) W.fl = first;
+  }
 }
 
 // Gen::gather_len (decode_general.rs:4260-4341) into W.above / W.left / W.tl.
-__device__ void gi_gather_len(const vvcg_gen_intra_state& S, int c, bool luma, int x, int y, int top_len,
+__device__ void gi_gather_len(const Grp& g, const vvcg_gen_intra_state& S, int c, bool luma, int x, int y, int top_len,
                               int left_len, GiWs& W) {
-  const int lane = threadIdx.x & 31;
   const int pw = c ? (int)S.width >> 1 : (int)S.width, ph = c ? (int)S.height >> 1 : (int)S.height;
   const int d = 1 << (S.bit_depth - 1);
-  int ft, fl;
-  gi_fill_side(S, c, top_len, W.above,
-               [&](int k) { return y > 0 && x + k < pw && gi_decoded(S, luma, x + k, y - 1); },
-               [&](int k, int* px, int* py) { *px = x + k; *py = y - 1; }, &ft);
-  gi_fill_side(S, c, left_len, W.left,
-               [&](int k) { return x > 0 && y + k < ph && gi_decoded(S, luma, x - 1, y + k); },
-               [&](int k, int* px, int* py) { *px = x - 1; *py = y + k; }, &fl);
+  // the corner's loads go out with the sides'
+  const int tlv = x > 0 && y > 0 ? gi_get(S, c, x - 1, y - 1) : 0;
   const bool tl = x > 0 && y > 0 && gi_decoded(S, luma, x - 1, y - 1);
+  gi_fill(g, S, c, top_len, left_len, W,
+          [&](int k) { return y > 0 && x + k < pw && gi_decoded(S, luma, x + k, y - 1); },
+          [&](int k, int* px, int* py) { *px = x + k; *py = y - 1; },
+          [&](int k) { return x > 0 && y + k < ph && gi_decoded(S, luma, x - 1, y + k); },
+          [&](int k, int* px, int* py) { *px = x - 1; *py = y + k; });
+  g.sync();
+  const int ft = W.ft, fl = W.fl;
   const bool any = ft >= 0 || fl >= 0 || tl;
   // positions with nothing available before them: first_top / first_left / dc
   const int fa = ft >= 0 ? ft : fl >= 0 ? fl : d, flb = fl >= 0 ? fl : ft >= 0 ? ft : d;
-  for (int k = lane; k < top_len; k += 32)
+  for (int k = g.tid; k < top_len; k += g.n)
     if (!any) W.above[k] = (int16_t)d; else if (W.above[k] < 0) W.above[k] = (int16_t)fa;
-  for (int k = lane; k < left_len; k += 32)
+  for (int k = g.tid; k < left_len; k += g.n)
     if (!any) W.left[k] = (int16_t)d; else if (W.left[k] < 0) W.left[k] = (int16_t)flb;
-  if (lane == 0) W.tl = tl ? gi_get(S, c, x - 1, y - 1) : fa;
-  __syncwarp();
+  if (g.tid == 0) W.tl = tl ? tlv : fa;
+  g.sync();
 }
 
 // MrlRefSamples::from_ref_samples (predict.rs:1058-1075) of W.above / W.left.
-__device__ void gi_rows_from_refs(int top_len, int left_len, GiWs& W) {
-  const int lane = threadIdx.x & 31;
-  for (int i = lane; i < top_len + 5; i += 32) W.rowa[i] = i == 0 ? (int16_t)W.tl : W.above[min(i - 1, top_len - 1)];
-  for (int i = lane; i < left_len + 5; i += 32) W.rowl[i] = i == 0 ? (int16_t)W.tl : W.left[min(i - 1, left_len - 1)];
-  if (lane == 0) {
+__device__ void gi_rows_from_refs(const Grp& g, int top_len, int left_len, GiWs& W) {
+  for (int i = g.tid; i < top_len + 5; i += g.n) W.rowa[i] = i == 0 ? (int16_t)W.tl : W.above[min(i - 1, top_len - 1)];
+  for (int i = g.tid; i < left_len + 5; i += g.n) W.rowl[i] = i == 0 ? (int16_t)W.tl : W.left[min(i - 1, left_len - 1)];
+  if (g.tid == 0) {
     W.nrowa = top_len + 5;
     W.nrowl = left_len + 5;
     W.off = 0;
   }
-  __syncwarp();
+  g.sync();
 }
 
 // Gen::gather_mrl (decode_general.rs:4542-4632) into W.rowa / W.rowl.
-__device__ void gi_gather_mrl(const vvcg_gen_intra_state& S, int x, int y, int w, int h, int mrl, GiWs& W) {
-  const int lane = threadIdx.x & 31;
+__device__ void gi_gather_mrl(const Grp& g, const vvcg_gen_intra_state& S, int x, int y, int w, int h, int mrl, GiWs& W) {
   const int d = 1 << (S.bit_depth - 1), off = 1 + mrl, al = 2 * w, ll = 2 * h;
-  int ft, fl;
-  gi_fill_side(S, 0, al, W.above,
-               [&](int k) { return y >= off && x + k < (int)S.width && gi_decoded(S, true, x + k, y - off); },
-               [&](int k, int* px, int* py) { *px = x + k; *py = y - off; }, &ft);
-  gi_fill_side(S, 0, ll, W.left,
-               [&](int k) { return x >= off && y + k < (int)S.height && gi_decoded(S, true, x - off, y + k); },
-               [&](int k, int* px, int* py) { *px = x - off; *py = y + k; }, &fl);
+  gi_fill(g, S, 0, al, ll, W,
+          [&](int k) { return y >= off && x + k < (int)S.width && gi_decoded(S, true, x + k, y - off); },
+          [&](int k, int* px, int* py) { *px = x + k; *py = y - off; },
+          [&](int k) { return x >= off && y + k < (int)S.height && gi_decoded(S, true, x - off, y + k); },
+          [&](int k, int* px, int* py) { *px = x - off; *py = y + k; });
   const bool tl = x >= off && y >= off && gi_decoded(S, true, x - off, y - off);
+  g.sync();
+  const int ft = W.ft, fl = W.fl;
   const int fa = ft >= 0 ? ft : fl >= 0 ? fl : d, flb = fl >= 0 ? fl : ft >= 0 ? ft : d;
   const int fb = fa;  // the corner fallback: first_top, first_left, dc
-  for (int i = lane; i < al + off + 4; i += 32) {
+  for (int i = g.tid; i < al + off + 4; i += g.n) {
     int v;
     if (i < off) {
       v = tl ? gi_get(S, 0, x - off + i, y - off) : fb;
@@ -195,7 +230,7 @@ __device__ void gi_gather_mrl(const vvcg_gen_intra_state& S, int x, int y, int w
     }
     W.rowa[i] = (int16_t)v;
   }
-  for (int i = lane; i < ll + off + 4; i += 32) {
+  for (int i = g.tid; i < ll + off + 4; i += g.n) {
     int v;
     if (i < off) {
       v = tl ? gi_get(S, 0, x - off, y - off + i) : fb;
@@ -205,35 +240,34 @@ __device__ void gi_gather_mrl(const vvcg_gen_intra_state& S, int x, int y, int w
     }
     W.rowl[i] = (int16_t)v;
   }
-  if (lane == 0) {
+  if (g.tid == 0) {
     W.nrowa = al + off + 4;
     W.nrowl = ll + off + 4;
     W.off = mrl;
   }
-  __syncwarp();
+  g.sync();
 }
 
 // predict_angular_with_params_bd (predict.rs:1776-1958) from W.rowa / W.rowl
 // with reference line mri; sink(i, v) per sample (raster of the w x h block).
 template <class Sink>
-__device__ void gi_angular(const GiAng& P, int w, int h, bool luma, int mri, int bd, GiWs& W, Sink sink) {
-  const int lane = threadIdx.x & 31;
+__device__ void gi_angular(const Grp& g, const GiAng& P, int w, int h, bool luma, int mri, int bd, GiWs& W, Sink sink) {
   const int def = 1 << (bd - 1), maxv = (1 << bd) - 1;
   const int base = max(h, w) + 4;
   const int len = base + 2 * max(w, h) + 2 * max(P.ref_w, P.ref_h) + 64;
   const int na = W.nrowa, nl = W.nrowl;
   const int a_hi = P.angle < 0 ? w + 1 + mri : P.ref_w + mri;
   const int l_hi = P.angle < 0 ? h + 1 + mri : P.ref_h + mri;
-  for (int i = lane; i < len; i += 32) {
+  for (int i = g.tid; i < len; i += g.n) {
     const int x = i - base;
     W.ra[i] = (x >= 0 && x <= a_hi) ? W.rowa[min(x, na - 1)] : (int16_t)def;
     W.rl[i] = (x >= 0 && x <= l_hi) ? W.rowl[min(x, nl - 1)] : (int16_t)def;
   }
-  __syncwarp();
+  g.sync();
   const bool ver = P.ver;
   if (P.angle < 0) {
     const int side = ver ? h : w;
-    for (int k = -side + lane; k <= -1; k += 32) {
+    for (int k = -side + g.tid; k <= -1; k += g.n) {
       const int proj = min((-k * P.abs_inv + 256) >> 9, side);
       if (ver)
         W.ra[base + k] = W.rl[base + proj];
@@ -247,9 +281,9 @@ __device__ void gi_angular(const GiAng& P, int w, int h, bool luma, int mri, int
     const int ref_length = ver ? P.ref_w : P.ref_h;
     int16_t* r = ver ? W.ra : W.rl;
     const int16_t v = r[base + ref_length + mri];
-    for (int z = 1 + lane; z <= max_index; z += 32) r[base + ref_length + mri + z] = v;
+    for (int z = 1 + g.tid; z <= max_index; z += g.n) r[base + ref_length + mri + z] = v;
   }
-  __syncwarp();
+  g.sync();
   const int mb = base + mri, sb = base + mri;
   const int16_t* rm = ver ? W.ra : W.rl;
   const int16_t* rs = ver ? W.rl : W.ra;
@@ -258,8 +292,9 @@ __device__ void gi_angular(const GiAng& P, int w, int h, bool luma, int mri, int
   const int pscale = max(P.scale, 0);
   const int plimit = min(3 << pscale, ww);
   const int scale0 = (floor_log2(ww) + floor_log2(wh) - 2) >> 2;
-  for (int i = lane; i < w * h; i += 32) {
-    const int r = i / w, c = i - r * w;
+  const int lgw = floor_log2(w);
+  for (int i = g.tid; i < w * h; i += g.n) {
+    const int r = i >> lgw, c = i & (w - 1);
     const int x = ver ? c : r, y = ver ? r : c;
     int v;
     if (P.angle == 0) {
@@ -303,12 +338,12 @@ __device__ void gi_angular(const GiAng& P, int w, int h, bool luma, int mri, int
     }
     sink(i, v);
   }
-  __syncwarp();
+  g.sync();
 }
 
 // Planar / DC (predict.rs:1688-1736) on W.ba / W.bl / W.btl, PDPC when asked.
 template <class Sink>
-__device__ void gi_planar_dc(bool planar, int w, int h, bool pdpc, GiWs& W, Sink sink) {
+__device__ void gi_planar_dc(const Grp& g, bool planar, int w, int h, bool pdpc, GiWs& W, Sink sink) {
   const int lane = threadIdx.x & 31;
   const int lw = floor_log2(w), lh = floor_log2(h);
   const int tr = W.ba[w], bl = W.bl[h];
@@ -324,7 +359,7 @@ __device__ void gi_planar_dc(bool planar, int w, int h, bool pdpc, GiWs& W, Sink
     dcv = (s + (denom >> 1)) >> floor_log2(denom);
   }
   const int sc = max(lw + lh - 2, 0) >> 2;
-  for (int i = lane; i < w * h; i += 32) {
+  for (int i = g.tid; i < w * h; i += g.n) {
     const int y = i >> lw, x = i & (w - 1);
     int v;
     if (planar) {
@@ -340,19 +375,18 @@ __device__ void gi_planar_dc(bool planar, int w, int h, bool pdpc, GiWs& W, Sink
     }
     sink(i, v);
   }
-  __syncwarp();
+  g.sync();
 }
 
 // RefSamples::filtered (predict.rs:1233-1267) of `n` above / left samples
 // from src arrays (with top-left) into W.ba / W.bl / W.btl.
-__device__ void gi_filter_into_base(const int16_t* sa, const int16_t* sl, int tlv, int na, int nl, GiWs& W) {
-  const int lane = threadIdx.x & 31;
-  for (int j = lane; j < na; j += 32)
+__device__ void gi_filter_into_base(const Grp& g, const int16_t* sa, const int16_t* sl, int tlv, int na, int nl, GiWs& W) {
+  for (int j = g.tid; j < na; j += g.n)
     W.ba[j] = j + 1 < na ? (int16_t)(((j == 0 ? tlv : sa[j - 1]) + 2 * sa[j] + sa[j + 1] + 2) >> 2) : sa[j];
-  for (int j = lane; j < nl; j += 32)
+  for (int j = g.tid; j < nl; j += g.n)
     W.bl[j] = j + 1 < nl ? (int16_t)(((j == 0 ? tlv : sl[j - 1]) + 2 * sl[j] + sl[j + 1] + 2) >> 2) : sl[j];
-  if (lane == 0) W.btl = (2 * tlv + sa[0] + sl[0] + 2) >> 2;
-  __syncwarp();
+  if (g.tid == 0) W.btl = (2 * tlv + sa[0] + sl[0] + 2) >> 2;
+  g.sync();
 }
 
 // derive_cclm_params_from_4_samples (predict.rs:2088-2177); sl / sc of count
@@ -410,7 +444,7 @@ __device__ __forceinline__ void gi_cclm_params(int* sl, int* sc, int cnt, int bd
 
 // Gen::cclm_predict (decode_general.rs:4372-4537); mode 0 LM, 1 LM-L, 2 LM-T.
 template <class Sink>
-__device__ void gi_cclm(const vvcg_gen_intra_state& S, int comp, int mode, int xc, int yc, int w, int h, Sink sink) {
+__device__ void gi_cclm(const Grp& g, const vvcg_gen_intra_state& S, int comp, int mode, int xc, int yc, int w, int h, Sink sink) {
   const int lane = threadIdx.x & 31;
   const int bd = S.bit_depth, mid = 1 << (bd - 1), maxv = (1 << bd) - 1;
   const int xtb = xc * 2, ytb = yc * 2;
@@ -486,8 +520,9 @@ __device__ void gi_cclm(const vvcg_gen_intra_state& S, int comp, int mode, int x
   }
   int a = 0, b = mid, shift = 0;
   if (count > 0) gi_cclm_params(sl, sc, count, bd, &a, &b, &shift);
-  for (int i = lane; i < w * h; i += 32) {
-    const int y = i / w, x = i - y * w;
+  const int lgw = floor_log2(w);
+  for (int i = g.tid; i < w * h; i += g.n) {
+    const int y = i >> lgw, x = i & (w - 1);
     int v = mid;
     if (count > 0) {
       const int lx = 2 * x, ly = 2 * y;
@@ -498,92 +533,92 @@ __device__ void gi_cclm(const vvcg_gen_intra_state& S, int comp, int mode, int x
     }
     sink(i, v);
   }
-  __syncwarp();
+  g.sync();
 }
 
-// The prediction of one request, by the calling warp: emit(i, v) per sample
+// The prediction of one request, by a group: emit(i, v) per sample
 // (i: raster index in the w x h block), once every reference is in W.
 template <class Emit>
-__device__ void gi_predict_emit(const vvcg_gen_intra_state& S, const vvcg_gen_intra_req& R, GiWs& W, Emit emit) {
-  const int lane = threadIdx.x & 31;
+__device__ void gi_predict_emit(const Grp& g, const vvcg_gen_intra_state& S, const vvcg_gen_intra_req& R, GiWs& W, Emit emit) {
   const int bd = S.bit_depth;
   if (R.comp == 0) {
     // the 4-wide region of narrow vertical ISP sub-partitions
     const bool region = R.isp == VVCG_ISP_VER && (R.cu_w == 4 || (R.cu_w == 8 && R.cu_h > 4));
     const int px = region ? R.cu_x + ((R.x - R.cu_x) / 4) * 4 : R.x;
     const int pw = region ? 4 : R.w, ph = R.h, col0 = R.x - px;
+    const int lgw = floor_log2(pw);
     auto put = [&](int i, int v) {
-      const int yy = i / pw, xx = i - yy * pw - col0;
+      const int yy = i >> lgw, xx = (i & (pw - 1)) - col0;
       if (xx >= 0 && xx < R.w) emit(yy * R.w + xx, v);
     };
     if (R.bdpcm) {
-      gi_gather_len(S, 0, true, px, R.y, 2 * pw, 2 * ph, W);
-      for (int i = lane; i < pw * ph; i += 32) {
-        const int yy = i / pw, xx = i - yy * pw;
+      gi_gather_len(g, S, 0, true, px, R.y, 2 * pw, 2 * ph, W);
+      for (int i = g.tid; i < pw * ph; i += g.n) {
+        const int yy = i >> lgw, xx = i & (pw - 1);
         put(i, R.bdpcm == VVCG_BDPCM_VER ? W.above[xx] : W.left[yy]);
       }
-      __syncwarp();
+      g.sync();
       return;
     }
     const bool isp = R.isp != VVCG_ISP_NONE;
     const int mrl = min((int)R.mrl, 2);
     if (isp) {
-      gi_gather_len(S, 0, true, px, R.y, R.cu_w + pw, R.cu_h + ph, W);
-      gi_rows_from_refs(R.cu_w + pw, R.cu_h + ph, W);
+      gi_gather_len(g, S, 0, true, px, R.y, R.cu_w + pw, R.cu_h + ph, W);
+      gi_rows_from_refs(g, R.cu_w + pw, R.cu_h + ph, W);
     } else if (mrl == 0) {
-      gi_gather_len(S, 0, true, px, R.y, 2 * pw, 2 * ph, W);
-      gi_rows_from_refs(2 * pw, 2 * ph, W);
+      gi_gather_len(g, S, 0, true, px, R.y, 2 * pw, 2 * ph, W);
+      gi_rows_from_refs(g, 2 * pw, 2 * ph, W);
     } else {
-      gi_gather_mrl(S, px, R.y, pw, ph, mrl, W);
+      gi_gather_mrl(g, S, px, R.y, pw, ph, mrl, W);
     }
     const int off = W.off;
     const int mode = R.mode;
     if (mode <= 1) {
       const bool filt = mode == 0 && mrl == 0 && !isp && pw * ph > 32;
       if (filt) {
-        gi_filter_into_base(W.rowa + off + 1, W.rowl + off + 1, W.rowa[off], 2 * pw, 2 * ph, W);
+        gi_filter_into_base(g, W.rowa + off + 1, W.rowl + off + 1, W.rowa[off], 2 * pw, 2 * ph, W);
       } else {
-        for (int i = lane; i < 2 * pw; i += 32) W.ba[i] = W.rowa[off + 1 + i];
-        for (int i = lane; i < 2 * ph; i += 32) W.bl[i] = W.rowl[off + 1 + i];
-        __syncwarp();
+        for (int i = g.tid; i < 2 * pw; i += g.n) W.ba[i] = W.rowa[off + 1 + i];
+        for (int i = g.tid; i < 2 * ph; i += g.n) W.bl[i] = W.rowl[off + 1 + i];
+        g.sync();
       }
-      gi_planar_dc(mode == 0, pw, ph, mrl == 0 && pw >= 4 && ph >= 4, W, put);
+      gi_planar_dc(g, mode == 0, pw, ph, mrl == 0 && pw >= 4 && ph >= 4, W, put);
       return;
     }
     const GiAng P = gi_ang_params(min(mode, 66), pw, ph, R.cu_w, R.cu_h, true, mrl, isp);
     if (mrl == 0 && !isp && P.ref_filter) {
       // rows from the filtered base refs
-      gi_filter_into_base(W.rowa + 1, W.rowl + 1, W.rowa[0], 2 * pw, 2 * ph, W);
-      for (int i = lane; i < 2 * pw + 5; i += 32) W.rowa[i] = i == 0 ? (int16_t)W.btl : W.ba[min(i - 1, 2 * pw - 1)];
-      for (int i = lane; i < 2 * ph + 5; i += 32) W.rowl[i] = i == 0 ? (int16_t)W.btl : W.bl[min(i - 1, 2 * ph - 1)];
-      __syncwarp();
+      gi_filter_into_base(g, W.rowa + 1, W.rowl + 1, W.rowa[0], 2 * pw, 2 * ph, W);
+      for (int i = g.tid; i < 2 * pw + 5; i += g.n) W.rowa[i] = i == 0 ? (int16_t)W.btl : W.ba[min(i - 1, 2 * pw - 1)];
+      for (int i = g.tid; i < 2 * ph + 5; i += g.n) W.rowl[i] = i == 0 ? (int16_t)W.btl : W.bl[min(i - 1, 2 * ph - 1)];
+      g.sync();
     }
-    gi_angular(P, pw, ph, true, W.off, bd, W, put);  // the rows' reference line
+    gi_angular(g, P, pw, ph, true, W.off, bd, W, put);  // the rows' reference line
     return;
   }
   // chroma
   auto put = [&](int i, int v) { emit(i, v); };
   const int w = R.w, h = R.h;
   if (R.mode >= 81 && R.mode <= 83) {
-    gi_cclm(S, R.comp, R.mode - 81, R.x, R.y, w, h, put);
+    gi_cclm(g, S, R.comp, R.mode - 81, R.x, R.y, w, h, put);
     return;
   }
-  gi_gather_len(S, R.comp, false, R.x, R.y, 2 * w, 2 * h, W);
+  gi_gather_len(g, S, R.comp, false, R.x, R.y, 2 * w, 2 * h, W);
   if (R.mode <= 1) {
-    for (int i = lane; i < 2 * w; i += 32) W.ba[i] = W.above[i];
-    for (int i = lane; i < 2 * h; i += 32) W.bl[i] = W.left[i];
-    __syncwarp();
-    gi_planar_dc(R.mode == 0, w, h, w >= 4 && h >= 4, W, put);
+    for (int i = g.tid; i < 2 * w; i += g.n) W.ba[i] = W.above[i];
+    for (int i = g.tid; i < 2 * h; i += g.n) W.bl[i] = W.left[i];
+    g.sync();
+    gi_planar_dc(g, R.mode == 0, w, h, w >= 4 && h >= 4, W, put);
     return;
   }
-  gi_rows_from_refs(2 * w, 2 * h, W);
+  gi_rows_from_refs(g, 2 * w, 2 * h, W);
   const GiAng P = gi_ang_params(min((int)R.mode, 66), w, h, w, h, false, 0, false);
-  gi_angular(P, w, h, false, 0, bd, W, put);
+  gi_angular(g, P, w, h, false, 0, bd, W, put);
 }
 
 // The prediction of one request into out (w x h int16, row-major).
-__device__ void gi_predict(const vvcg_gen_intra_state& S, const vvcg_gen_intra_req& R, int16_t* out, GiWs& W) {
-  gi_predict_emit(S, R, W, [&](int i, int v) { out[i] = (int16_t)v; });
+__device__ void gi_predict(const Grp& g, const vvcg_gen_intra_state& S, const vvcg_gen_intra_req& R, int16_t* out, GiWs& W) {
+  gi_predict_emit(g, S, R, W, [&](int i, int v) { out[i] = (int16_t)v; });
 }
 
 __global__ void __launch_bounds__(kGiWarps * 32) k_gen_intra(const __grid_constant__ GenIntraArgs A) {
@@ -591,7 +626,7 @@ __global__ void __launch_bounds__(kGiWarps * 32) k_gen_intra(const __grid_consta
   const int warp = threadIdx.x >> 5;
   for (int q = blockIdx.x * kGiWarps + warp; q < A.n; q += gridDim.x * kGiWarps) {
     const vvcg_gen_intra_req R = A.reqs[q];
-    gi_predict(A.st, R, A.out + R.out_off, ws[warp]);
+    gi_predict(Grp{(int)threadIdx.x & 31, 32, 0}, A.st, R, A.out + R.out_off, ws[warp]);
   }
 }
 
@@ -617,7 +652,7 @@ struct GenReconArgs {
 __device__ void gi_recon_block(const vvcg_gen_intra_state& S, const vvcg_gen_intra_req& R, int16_t* pred,
                                const int16_t* res, GiWs& ws, int lane) {
   const int maxv = (1 << S.bit_depth) - 1;
-  gi_predict(S, R, pred, ws);
+  gi_predict(Grp{lane, 32, 0}, S, R, pred, ws);
   __syncwarp();
   uint16_t* pl = const_cast<uint16_t*>(S.plane[R.comp]);
   const int st = (int)S.stride[R.comp];
@@ -643,32 +678,33 @@ __device__ void gi_recon_block(const vvcg_gen_intra_state& S, const vvcg_gen_int
   __syncwarp();
 }
 
-// gi_recon_block without the prediction buffer: each predicted sample goes
-// straight into the plane with its residual added and clipped.
-__device__ void gi_recon_block_fused(const vvcg_gen_intra_state& S, const vvcg_gen_intra_req& R,
-                                     const int16_t* __restrict__ res, GiWs& ws, int lane) {
-  const int maxv = (1 << S.bit_depth) - 1;
-  uint16_t* pl = const_cast<uint16_t*>(S.plane[R.comp]);
+// gi_recon_block by a group and without the prediction buffer: each predicted
+// sample goes straight into the plane with its residual added and clipped.
+// Residual loads for the group's first samples go out before the references'.
+__device__ void gi_recon_block_fused(const Grp& g, const vvcg_gen_intra_state& S, const vvcg_gen_intra_req& R,
+                                     const int16_t* __restrict__ res, GiWs& ws) {
+  const int maxv = (1 << S.bit_depth) - 1, n = R.w * R.h, lw = floor_log2(R.w);
+  const int r0 = g.tid < n ? (int)__ldcs(res + g.tid) : 0;
+  uint16_t* pl = const_cast<uint16_t*>(S.plane[R.comp]) + (size_t)R.y * S.stride[R.comp] + R.x;
   const int st = (int)S.stride[R.comp];
-  gi_predict_emit(S, R, ws, [&](int i, int v) {
-    const int yy = i / R.w, xx = i - yy * R.w;
-    pl[(size_t)(R.y + yy) * st + R.x + xx] = (uint16_t)clampi(v + (int)res[i], 0, maxv);
+  gi_predict_emit(g, S, R, ws, [&](int i, int v) {
+    pl[(size_t)(i >> lw) * st + (i & (R.w - 1))] = (uint16_t)clampi(v + (i == g.tid ? r0 : (int)res[i]), 0, maxv);
   });
-  __syncwarp();
+  g.sync();
   if (R.comp == 0) {
     uint8_t* dm = const_cast<uint8_t*>(S.dec_y);
     const int cw = (int)S.width >> 2;
     const int x0 = R.x >> 2, x1 = min((R.x + R.w + 3) >> 2, cw), y0 = R.y >> 2;
     const int y1 = min((R.y + R.h + 3) >> 2, (int)S.height >> 2);
-    for (int i = lane; i < (x1 - x0) * (y1 - y0); i += 32)
+    for (int i = g.tid; i < (x1 - x0) * (y1 - y0); i += g.n)
       dm[(size_t)(y0 + i / (x1 - x0)) * cw + x0 + i % (x1 - x0)] = 1;
   } else {
     uint8_t* dm = const_cast<uint8_t*>(S.dec_c);
     const int cw = (int)S.width >> 1;
-    for (int i = lane; i < R.w * R.h; i += 32) dm[(size_t)(R.y + i / R.w) * cw + R.x + i % R.w] = 1;
+    for (int i = g.tid; i < n; i += g.n) dm[(size_t)(R.y + (i >> lw)) * cw + R.x + (i & (R.w - 1))] = 1;
   }
   __threadfence_block();
-  __syncwarp();
+  g.sync();
 }
 
 __global__ void __launch_bounds__(kGiWarps * 32) k_gen_intra_recon(const __grid_constant__ GenReconArgs A) {
@@ -681,32 +717,124 @@ __global__ void __launch_bounds__(kGiWarps * 32) k_gen_intra_recon(const __grid_
     }
 }
 
-// One dependency level of the general picture pass: each warp takes coding
-// units (groups of blocks in decode order) of the level, from any picture of
-// the batch, and reconstructs their blocks in order. The host puts a group
-// in a later level than every earlier group whose samples it may read and
-// every earlier group that may read its samples, so the decoded maps each
-// block sees are those of the picture's sequential decode.
-struct GenLevelArgs {
+// The intra reconstruction of the general picture pass: a persistent kernel
+// whose CTAs take the groups (coding units: blocks in decode order) of every
+// picture, level by level. The host puts a group in a later level of its
+// picture than every earlier group whose samples it may read and every earlier
+// group that may read its samples; a group starts when the picture's level
+// before its own is complete (a counter per picture and level, bounded wait),
+// so the decoded maps each block sees are those of the picture's sequential
+// decode. Groups are handed out in level order, so the groups a CTA waits for
+// are held by running CTAs.
+//
+// What bounds it is the chain of a picture's levels: a wait, the references'
+// round trip, the prediction, the stores and the release, once per block that a
+// group must do one after another. So the luma blocks take six warps, and Cb
+// and Cr a warp each beside them (CCLM after them); a chroma block never reads
+// another component's chroma or decoded map inside its own area. Groups of
+// another make-up (kGenInOrder) are done block by block.
+constexpr int kGenLuma = 192, kGenThreads = kGenLuma + 64;
+constexpr uint32_t kGenInOrder = 1u << 31;
+
+struct GenGroup {      // in hand-out order
+  uint32_t group, pic;
+  uint32_t wait_at;    // counter of the picture's level before (its complete value in wait_for; 0: no wait)
+  uint32_t wait_for;
+  uint32_t done_at;    // counter of its own level, | kGenInOrder
+};
+
+struct GenPassArgs {
   const vvcg_gen_intra_state* states;  // per picture
   const vvcg_gen_intra_req* reqs;      // all blocks of the batch
   const uint32_t* group_first;         // per group: first block; group_first[g + 1] ends it
-  const uint32_t* group_pic;           // per group: picture
-  const uint32_t* level_groups;        // the groups of this level
-  uint32_t n;
+  const GenGroup* groups;
+  uint32_t n, spin_limit;
+  uint32_t* ctrl;                      // [0] hand-out counter, [1] status
+  uint32_t* done;                      // groups finished per picture and level
   const int16_t* res;                  // residuals at out_off (zero where uncoded)
-  int16_t* pred;                       // predictions at out_off
 };
 
-__global__ void __launch_bounds__(kGiWarps * 32) k_gen_recon_level(const __grid_constant__ GenLevelArgs A) {
-  __shared__ GiWs ws[kGiWarps];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (uint32_t i = blockIdx.x * kGiWarps + warp; i < A.n; i += gridDim.x * kGiWarps) {
-    const uint32_t g = A.level_groups[i];
-    const vvcg_gen_intra_state& S = A.states[A.group_pic[g]];
-    for (uint32_t q = A.group_first[g]; q < A.group_first[g + 1]; q++) {
-      const vvcg_gen_intra_req R = A.reqs[q];
-      gi_recon_block_fused(S, R, A.res + R.out_off, ws[warp], lane);
+constexpr int kGenReqs = 16;  // a group's first blocks, fetched before its wait
+
+__global__ void __launch_bounds__(kGenThreads, 3) k_gen_recon(const __grid_constant__ GenPassArgs A) {
+  __shared__ GiWs ws[3];
+  __shared__ __align__(16) vvcg_gen_intra_state s_state;
+  __shared__ vvcg_gen_intra_req s_req[kGenReqs];
+  __shared__ GenGroup s_group;
+  __shared__ uint32_t s_item, s_first[2];
+  const int t = threadIdx.x, lane = t & 31;
+  uint32_t pic = 0xFFFFFFFFu;
+  for (;;) {
+    // the next group, its picture and its blocks, before the wait
+    if (t < 32) {
+      uint32_t it = 0;
+      if (lane == 0) it = atomicAdd(A.ctrl, 1u);
+      it = __shfl_sync(0xffffffffu, it, 0);
+      if (it < A.n) {
+        if (lane < (int)(sizeof(GenGroup) / 4))
+          reinterpret_cast<uint32_t*>(&s_group)[lane] = reinterpret_cast<const uint32_t*>(&A.groups[it])[lane];
+        __syncwarp();
+        if (lane < 2) s_first[lane] = A.group_first[s_group.group + lane];
+      }
+      if (lane == 0) s_item = it;
+    }
+    __syncthreads();
+    if (s_item >= A.n) break;
+    const GenGroup G = s_group;
+    const uint32_t q0 = s_first[0], nq = s_first[1] - q0;
+    const bool in_order = (G.done_at & kGenInOrder) != 0;
+    constexpr int kReqWords = sizeof(vvcg_gen_intra_req) / 4;
+    for (int i = t; i < (int)min(nq, (uint32_t)kGenReqs) * kReqWords; i += kGenThreads)
+      reinterpret_cast<uint32_t*>(s_req)[i] = reinterpret_cast<const uint32_t*>(A.reqs + q0)[i];
+    if (pic != G.pic) {
+      pic = G.pic;
+      if (t < (int)(sizeof(vvcg_gen_intra_state) / 4))
+        reinterpret_cast<uint32_t*>(&s_state)[t] = reinterpret_cast<const uint32_t*>(&A.states[pic])[t];
+    }
+    if (t == 0 && G.wait_for) {
+      const uint32_t* c = A.done + G.wait_at;
+      bool ok = (ld_acquire(A.ctrl + 1) & kStatusTimeout) == 0;  // a wait gave up: the result is void
+      for (uint32_t it = 0; ok && ld_relaxed(c) < G.wait_for; it++) {
+        if (it >= A.spin_limit) {
+          atomicOr(A.ctrl + 1, kStatusTimeout);
+          ok = false;
+        } else if (it >= 64) {
+          __nanosleep(100);
+        }
+      }
+      fence_acq_rel();  // once: an acquire at every poll would drop the SM's L1 each time
+    }
+    __syncthreads();
+    const vvcg_gen_intra_state& S = s_state;
+    auto req = [&](uint32_t k) -> const vvcg_gen_intra_req& { return k < kGenReqs ? s_req[k] : A.reqs[q0 + k]; };
+    if (in_order) {
+      const Grp all{t, kGenThreads, 2};
+      for (uint32_t k = 0; k < nq; k++) {
+        const vvcg_gen_intra_req& R = req(k);
+        gi_recon_block_fused(all, S, R, A.res + R.out_off, ws[0]);
+      }
+    } else {
+      // luma blocks first, then at most one Cb and one Cr block: beside the
+      // luma, or (CCLM) after it by half the CTA each
+      const uint32_t last = nq - 1;
+      const bool cclm = req(last).comp && req(last).mode >= 81 && req(last).mode <= 83;
+      const bool cclm0 = nq > 1 && req(last - 1).comp && req(last - 1).mode >= 81 && req(last - 1).mode <= 83;
+      for (int phase = 0; phase < (cclm || cclm0 ? 2 : 1); phase++) {
+        if (phase) __syncthreads();
+        const int comp = phase ? 1 + (t >> 7) : (t < kGenLuma ? 0 : (t < kGenLuma + 32 ? 1 : 2));
+        const Grp g = phase ? Grp{t & 127, 128, comp} : (comp == 0 ? Grp{t, kGenLuma, 1} : Grp{lane, 32, 0});
+        for (uint32_t k = comp == 0 || nq < 2 ? 0 : nq - 2; k < nq; k++) {
+          const vvcg_gen_intra_req& R = req(k);
+          if (R.comp != comp) continue;
+          const bool late = R.comp && R.mode >= 81 && R.mode <= 83;
+          if (late == (phase == 1)) gi_recon_block_fused(g, S, R, A.res + R.out_off, ws[comp]);
+        }
+      }
+    }
+    __syncthreads();
+    if (t == 32 * 7) {  // not the warp that fetches and polls next
+      __threadfence();
+      atomicAdd(A.done + (G.done_at & ~kGenInOrder), 1u);
     }
   }
 }

@@ -4,9 +4,9 @@
 // defined there).
 //
 // Per run: the residual slots are cleared and every coded block's residual
-// is computed by the size-binned TU kernels; the intra reconstruction runs
-// level by level (k_gen_recon_level), each level a launch over the groups of
-// every picture that have no dependency left; then per picture the general
+// is computed by the size-binned TU kernels; the intra reconstruction
+// (k_gen_recon, one persistent launch) takes the groups of every picture level
+// by level; then per picture the general
 // deblocking (two launches), SAO (one per component) and ALF (two launches).
 //
 // Dependency levels (host, at prepare): the groups of a picture are visited
@@ -39,8 +39,9 @@ struct GenPass {
   std::vector<uint32_t> level_start;  // levels + 1 offsets into the level-ordered groups
   uint32_t tu_count[kTuBins] = {0, 0, 0};
   uint64_t slot_count = 0, maps_bytes = 0;
-  DevBuf planes, maps, states, reqs, tus, tu_idx, group_first, group_pic, level_groups, levels, res, pred, cells,
-      ccells, sao, alf_ctus, alf_params;
+  uint32_t num_work = 0, num_counters = 0;  // groups with blocks; picture levels
+  DevBuf planes, maps, states, reqs, tus, tu_idx, group_first, work, sync, levels, res, cells, ccells, sao, alf_ctus,
+      alf_params;  // sync: hand-out counter, status, then the level counters
   std::vector<DbkGenArgs> dbk;          // per picture (pictures without deblocking: unused)
   std::vector<SaoBoundedPass> sao_pass;  // 3 per picture with SAO
   std::vector<AlfGenPass> alf_pass;      // per picture with ALF
@@ -55,8 +56,8 @@ struct GenPass {
   }
   void release() {
     drop_graph();
-    for (DevBuf* b : {&planes, &maps, &states, &reqs, &tus, &tu_idx, &group_first, &group_pic, &level_groups, &levels,
-                      &res, &pred, &cells, &ccells, &sao, &alf_ctus, &alf_params})
+    for (DevBuf* b : {&planes, &maps, &states, &reqs, &tus, &tu_idx, &group_first, &work, &sync, &levels, &res, &cells,
+                      &ccells, &sao, &alf_ctus, &alf_params})
       b->release();
   }
 };
@@ -308,11 +309,42 @@ vvcg_status vvcg_gen_prepare(vvcg_ctx* ctx, const vvcg_gen_batch* b) {
   for (uint32_t g = 0; g < b->num_groups; g++)
     if (group_level[g]) G.level_start[group_level[g]]++;  // counts at [level]
   for (uint32_t l = 1; l <= max_level; l++) G.level_start[l] += G.level_start[l - 1];
-  std::vector<uint32_t> level_groups(G.level_start[max_level]);
+  // the groups in level order, each with the counters of its picture's levels:
+  // one per level, from counter_at[picture] on
+  std::vector<GenGroup> work(G.level_start[max_level]);
   {
-    std::vector<uint32_t> at(G.level_start.begin(), G.level_start.end() - 1);  // level L starts at [L - 1]
+    std::vector<uint32_t> top(np, 0), counter_at(np, 0), count;
     for (uint32_t g = 0; g < b->num_groups; g++)
-      if (group_level[g]) level_groups[at[group_level[g] - 1]++] = g;
+      if (group_level[g]) top[group_pic[g]] = std::max(top[group_pic[g]], group_level[g]);
+    uint32_t n = 0;
+    for (uint32_t i = 0; i < np; i++) {
+      counter_at[i] = n;
+      n += top[i];
+    }
+    count.assign(n, 0);
+    for (uint32_t g = 0; g < b->num_groups; g++)
+      if (group_level[g]) count[counter_at[group_pic[g]] + group_level[g] - 1]++;
+    std::vector<uint32_t> at(G.level_start.begin(), G.level_start.end() - 1);  // level L starts at [L - 1]
+    for (uint32_t g = 0; g < b->num_groups; g++) {
+      const uint32_t lv = group_level[g];
+      if (!lv) continue;
+      // luma blocks, then at most one Cb and one Cr block of the same area
+      const uint32_t q0 = b->group_first[g], q1 = b->group_first[g + 1];
+      uint32_t q = q0;
+      while (q < q1 && reqs[q].comp == 0) q++;
+      bool split = true;
+      const uint32_t nc = q1 - q;
+      if (nc == 1) split = reqs[q].comp == 1 || reqs[q].comp == 2;
+      if (nc == 2)
+        split = reqs[q].comp == 1 && reqs[q + 1].comp == 2 && reqs[q].x == reqs[q + 1].x &&
+                reqs[q].y == reqs[q + 1].y && reqs[q].w == reqs[q + 1].w && reqs[q].h == reqs[q + 1].h;
+      if (nc > 2) split = false;
+      const uint32_t c = counter_at[group_pic[g]] + lv - 1;
+      work[at[lv - 1]++] = GenGroup{g, group_pic[g], lv > 1 ? c - 1 : 0, lv > 1 ? count[c - 1] : 0,
+                                    c | (split ? 0 : kGenInOrder)};
+    }
+    G.num_work = (uint32_t)work.size();
+    G.num_counters = n;
   }
 
   // -- deblocking maps (mark_tu over each picture's blocks in decode order) --
@@ -351,8 +383,9 @@ vvcg_status vvcg_gen_prepare(vvcg_ctx* ctx, const vvcg_gen_batch* b) {
   if ((st = gen_upload(ctx, G.tus, tus.data(), tus.size())) != VVCG_OK) return st;
   if ((st = gen_upload(ctx, G.tu_idx, tu_idx.data(), tu_idx.size())) != VVCG_OK) return st;
   if ((st = gen_upload(ctx, G.group_first, b->group_first, (size_t)b->num_groups + 1)) != VVCG_OK) return st;
-  if ((st = gen_upload(ctx, G.group_pic, group_pic.data(), group_pic.size())) != VVCG_OK) return st;
-  if ((st = gen_upload(ctx, G.level_groups, level_groups.data(), level_groups.size())) != VVCG_OK) return st;
+  if ((st = gen_upload(ctx, G.work, work.data(), work.size())) != VVCG_OK) return st;
+  CK(G.sync.reserve((2 + (size_t)G.num_counters) * sizeof(uint32_t)), "cudaMalloc");
+  CK(cudaMemsetAsync(G.sync.p, 0, (2 + (size_t)G.num_counters) * sizeof(uint32_t), ctx->stream), "clear counters");
   if ((st = gen_upload(ctx, G.levels, b->levels, b->num_levels)) != VVCG_OK) return st;
   if ((st = gen_upload(ctx, G.cells, cells.data(), cells.size())) != VVCG_OK) return st;
   if ((st = gen_upload(ctx, G.ccells, ccells.data(), ccells.size())) != VVCG_OK) return st;
@@ -360,7 +393,6 @@ vvcg_status vvcg_gen_prepare(vvcg_ctx* ctx, const vvcg_gen_batch* b) {
   if ((st = gen_upload(ctx, G.alf_ctus, b->alf_ctus, b->alf_ctus ? b->num_alf_ctus : 0)) != VVCG_OK) return st;
   if ((st = gen_upload(ctx, G.alf_params, b->alf_params, b->alf_params ? b->num_alf_params : 0)) != VVCG_OK) return st;
   CK(G.res.reserve(std::max<uint64_t>(1, b->slot_count) * sizeof(int16_t)), "cudaMalloc");
-  CK(G.pred.reserve(std::max<uint64_t>(1, b->slot_count) * sizeof(int16_t)), "cudaMalloc");
 
   // -- filter passes with device pointers ------------------------------------
   G.dbk.assign(np, DbkGenArgs{});
@@ -458,17 +490,14 @@ vvcg_status gen_enqueue(vvcg_ctx* ctx, uint32_t* n) {
     }
     first += cnt;
   }
-  const uint32_t levels = (uint32_t)G.level_start.size() - 1;
-  for (uint32_t l = 0; l < levels; l++) {
-    const uint32_t cnt = G.level_start[l + 1] - G.level_start[l];
-    if (!cnt) continue;
-    GenLevelArgs A{(const vvcg_gen_intra_state*)G.states.p, (const vvcg_gen_intra_req*)G.reqs.p,
-                   (const uint32_t*)G.group_first.p, (const uint32_t*)G.group_pic.p,
-                   (const uint32_t*)G.level_groups.p + G.level_start[l], cnt, (const int16_t*)G.res.p,
-                   (int16_t*)G.pred.p};
-    const uint32_t grid = std::min<uint32_t>((cnt + kGiWarps - 1) / kGiWarps, (uint32_t)ctx->num_sms * 8);
-    k_gen_recon_level<<<grid, kGiWarps * 32, 0, ctx->stream>>>(A);
-    CK(cudaGetLastError(), "intra level launch");
+  CK(cudaMemsetAsync(G.sync.p, 0, (2 + (size_t)G.num_counters) * sizeof(uint32_t), ctx->stream), "clear counters");
+  if (G.num_work) {
+    uint32_t* sync = (uint32_t*)G.sync.p;
+    GenPassArgs A{(const vvcg_gen_intra_state*)G.states.p, (const vvcg_gen_intra_req*)G.reqs.p,
+                  (const uint32_t*)G.group_first.p, (const GenGroup*)G.work.p, G.num_work, ctx->spin_limit, sync,
+                  sync + 2, (const int16_t*)G.res.p};
+    k_gen_recon<<<std::min<uint32_t>(G.num_work, (uint32_t)ctx->num_sms * 3), kGenThreads, 0, ctx->stream>>>(A);
+    CK(cudaGetLastError(), "intra launch");
     (*n)++;
   }
   size_t si = 0, ai = 0;
@@ -564,7 +593,12 @@ vvcg_status vvcg_gen_download(vvcg_ctx* ctx, const vvcg_plane_out* out) {
          "download");
     }
   }
+  uint32_t status = 0;
+  CK(cudaMemcpyAsync(&status, (const uint32_t*)G.sync.p + 1, sizeof(status), cudaMemcpyDeviceToHost, ctx->stream),
+     "status");
   CK(cudaStreamSynchronize(ctx->stream), "download");
+  if (status & kStatusTimeout)
+    return fail(ctx, VVCG_TIMEOUT, "a wait for a dependency level gave up after %u polls", ctx->spin_limit);
   return VVCG_OK;
 }
 
