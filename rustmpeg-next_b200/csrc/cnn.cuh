@@ -3,16 +3,17 @@
 // decision depends on lambda) -> conv 3x3 2->32 + ReLU -> 3 x (conv 3x3
 // 32->32 + ReLU) -> global average -> 67 intra-mode logits and 6 split logits.
 //
-// Forward: one CTA per block (persistent over blocks). The block's
-// activations stay in shared memory as two ping-pong images of 34 x 34
-// pixels (a zero halo around 32 x 32) in four planes of 8 channels, 16 bytes
-// per pixel, so each layer's 3x3 convolution is 144 tcgen05 MMAs
-// (M = 128 pixels, N = 32 output channels, K = 16 input channels of one tap)
-// whose A operand points straight into the image: the 8 rows of a core
-// matrix are 8 neighbouring pixels of an image row (16 B apart), SBO steps
-// one image row, LBO one channel plane, and a tap is an address offset. The
-// 8 tiles of a layer accumulate in 256 TMEM columns; 8 warps read them back,
-// add the bias, apply ReLU and write the next image (or the average).
+// Forward: two blocks at a time per CTA, each with its own half of the
+// threads, image and TMEM (k_cnn_forward). A block's activations stay in
+// shared memory as one image of 34 x 34 pixels (a zero halo around 32 x 32)
+// in four planes of 8 channels, 16 bytes per pixel, so each layer's 3x3
+// convolution is 144 tcgen05 MMAs (M = 128 pixels, N = 32 output channels,
+// K = 16 input channels of one tap) whose A operand points straight into the
+// image: the 8 rows of a core matrix are 8 neighbouring pixels of an image
+// row (16 B apart), SBO steps one image row, LBO one channel plane, and a tap
+// is an address offset. The 8 tiles of a layer accumulate in 256 TMEM
+// columns; 8 warps read them back, add the bias, apply ReLU and write the
+// image again (or the average): the layer's MMAs are done with it by then.
 // The first layer (two input channels) runs on the CUDA cores.
 #pragma once
 #include "umma.cuh"
@@ -31,19 +32,81 @@ constexpr int kOffWs = kOffBi + kCnnModes, kOffBs = kOffWs + kCnnSplits * kCnnCh
 constexpr int kCnnParams = kOffBs + kCnnSplits;  // 30761
 
 constexpr int kImgW = 34;                 // 32 + halo
-constexpr int kPlane = kImgW * kImgW * 16;  // one plane of 8 channels, bytes
-constexpr int kImg = 4 * kPlane;            // 73984
+// One plane of 8 channels, bytes. The 16 bytes of padding spread the four
+// planes over the banks: layer 1 stores 4 bytes of every plane in two rows at
+// once (four-way conflicts without them).
+constexpr int kPlane = kImgW * kImgW * 16 + 16;
+constexpr int kImg = 4 * kPlane;
 constexpr int kPackL = 36 * 32 * 16;        // packed bf16 weights of one layer: [tap*4 + ci/8][co][ci%8]
 constexpr int kCnnThreads = 256;
 constexpr uint32_t kCnnIdesc = umma_idesc_bf16(128, 32);
-constexpr int kCnnMisc = (576 + 32 + 96 + 8 * 32 + 1024 + 32) * 4;
-constexpr int kCnnSmem = 2 * kImg + 3 * kPackL + kCnnMisc + 64;
+constexpr int kCnnGroups = 2;                   // blocks in flight per CTA of the forward pass
+constexpr int kHeadPitch = kCnnCh + 1;          // head weights by row, one bank apart
+constexpr int kXPad = 34 * 34;                  // the input zero-padded by one pixel
+constexpr int kCnnGroupF = kXPad + 8 * 32 + 32;  // floats of one group: input, partial averages, average
+constexpr int kCnnMisc = (576 + 32 + 96 + kCnnOut * kHeadPitch + 76 - kCnnOut % 4 + kCnnGroups * kCnnGroupF) * 4;
+constexpr int kCnnSmem = kCnnGroups * kImg + 3 * kPackL + kCnnMisc + 64;
+static_assert(kCnnSmem <= 227 * 1024, "forward shared memory");
 
 __device__ __forceinline__ uint16_t f2bf(float f) {  // round to nearest even
   const uint32_t u = __float_as_uint(f);
   return (uint16_t)((u + 0x7FFFu + ((u >> 16) & 1u)) >> 16);
 }
 __device__ __forceinline__ float bf2f(uint16_t b) { return __uint_as_float((uint32_t)b << 16); }
+// Two values to bf16, round to nearest even: the first in the low half. Equal
+// to f2bf for all but NaN.
+__device__ __forceinline__ uint32_t pack_bf2(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+// Two fp32 values in a register pair, and their fused multiply-adds (each
+// half rounds as fmaf does).
+__device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 f2_unpack(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// Sums v[c] over the warp for 32 channels c, into lane c: each step halves
+// the channels a lane carries (31 shuffles instead of 160; the additions pair
+// the same lanes, at distances 16, 8, 4, 2, 1, as a butterfly per channel).
+__device__ __forceinline__ float warp_sum32(float* v, int lane) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int c = 0; c < o; c++) {
+      const float send = up ? v[c] : v[c + o], keep = up ? v[c + o] : v[c];
+      v[c] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, o);
+    }
+  }
+  return v[0];
+}
+// Barriers of one group of kCnnThreads threads (the id in a register takes
+// all 16 barriers, which the one CTA of an SM can have).
+__device__ __forceinline__ void cnn_sync(int id) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kCnnThreads) : "memory");
+}
+__device__ __forceinline__ bool cnn_sync_and(int id, bool v) {
+  uint32_t r;
+  __syncwarp();
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, %2, %3, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"((uint32_t)v), "r"(id), "n"(kCnnThreads)
+      : "memory");
+  return r != 0;
+}
 
 // pack[layer][tap*4 + ci/8][co][ci%8] = bf16(W[co][ci][tap]) (forward), or with
 // flip the weights of the transposed convolution: [tap*4 + co/8][ci][co%8] =
@@ -79,149 +142,252 @@ struct CnnFwdArgs {
 
 // Issues the 144 MMAs of one 3x3 32->32 layer reading image `xin` with the
 // packed weights `w` into TMEM columns tile * 32, then (with commit) commits
-// to mbar.
+// to mbar; called behind elect_one(). The start address is the descriptor's
+// low field in 16-byte units (one pixel, and it never carries out of its 14
+// bits): every operand is a base descriptor plus an offset. Bound by the
+// operands' shared-memory reads, 4 KB of A and 1 KB of B per MMA at 128 B per
+// cycle (40 cycles; 41 measured).
 __device__ __forceinline__ void cnn_issue_layer(uint32_t tmem, uint32_t xin, uint32_t w, uint64_t* mbar,
                                                 bool commit = true) {
+  constexpr uint64_t kA = umma_desc(0, kPlane, kImgW * 16), kB = umma_desc(0, 512, 128);
+  const uint32_t a0 = (uint32_t)kA + (xin >> 4), b0 = (uint32_t)kB + (w >> 4);
+#pragma unroll 1
   for (int tile = 0; tile < 8; tile++) {
-    const int xg = tile & 3, yh = tile >> 2;
-    for (int tap = 0; tap < 9; tap++) {
-      const int dy = tap / 3, dx = tap % 3;
-      for (int h = 0; h < 2; h++) {
-        const uint32_t a = xin + 2 * h * kPlane + ((16 * yh + dy) * kImgW + 8 * xg + dx) * 16;
-        const uint32_t b = w + (tap * 4 + 2 * h) * 32 * 16;
-        umma_bf16(tmem + tile * 32, umma_desc(a, kPlane, kImgW * 16), umma_desc(b, 512, 128), kCnnIdesc,
-                  (tap | h) != 0);
-      }
-    }
+    const uint32_t at = a0 + (tile >> 2) * 16 * kImgW + (tile & 3) * 8;
+#pragma unroll
+    for (int tap = 0; tap < 9; tap++)
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+        umma_bf16(tmem + tile * 32, (kA >> 32 << 32) | (at + (tap / 3) * kImgW + tap % 3 + h * (2 * kPlane / 16)),
+                  (kB >> 32 << 32) | (b0 + (tap * 4 + 2 * h) * 32), kCnnIdesc, (tap | h) != 0);
   }
   if (commit) umma_commit(mbar);
 }
 
-__global__ void __launch_bounds__(kCnnThreads, 1) k_cnn_forward(const __grid_constant__ CnnFwdArgs A) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t* X0 = smem;
-  uint8_t* X1 = smem + kImg;
-  uint8_t* W = smem + 2 * kImg;
-  float* w1 = (float*)(W + 3 * kPackL);
-  float* b1 = w1 + 576;
-  float* bias = b1 + 32;   // [3][32]
-  float* gpart = bias + 96;  // [8 warps][32]
-  float* xin = gpart + 256;  // 32 x 32 input
-  float* gap = xin + 1024;   // [32]
-  uint64_t* mbar = (uint64_t*)(gap + 32);
-  uint32_t* tslot = (uint32_t*)(mbar + 1);
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+// The four input samples of thread t of a group (rows t / 32 + 8 k) of block
+// blk; false, with nothing read, for a block outside the plane.
+__device__ __forceinline__ bool cnn_load_px(const uint16_t* plane, int64_t stride, int width, int height,
+                                            const uint32_t* ctu_xy, int blk, int t, uint16_t* px) {
+  const uint32_t ux = ctu_xy[2 * blk], uy = ctu_xy[2 * blk + 1];
+  if (ux > (uint32_t)width - 32 || uy > (uint32_t)height - 32 || width < 32 || height < 32) return false;
+#pragma unroll
+  for (int k = 0; k < 4; k++) px[k] = plane[(int64_t)((int)uy + (t >> 5) + 8 * k) * stride + (int)ux + (t & 31)];
+  return true;
+}
 
-  // weights, zero images (the halos stay zero), TMEM, barrier
-  for (int i = t; i < 3 * kPackL / 16; i += kCnnThreads) ((uint4*)W)[i] = ((const uint4*)A.pack)[i];
-  for (int i = t; i < 2 * kImg / 16; i += kCnnThreads) ((uint4*)X0)[i] = make_uint4(0, 0, 0, 0);
-  for (int i = t; i < 576; i += kCnnThreads) w1[i] = A.params[kOffW1 + i];
-  if (t < 32) b1[t] = A.params[kOffB1 + t];
-  if (t < 96) bias[t] = A.params[cnn_off_b(2 + t / 32) + t % 32];
-  if (warp == 0) {
-    tmem_alloc(tslot, 256);
+// Layer 1 of one block on the CUDA cores: 16 lanes take a pair of channels
+// each (both in one packed fp32 operation) and the warp's halves two image
+// rows each, so the 36 weights of a thread stay in registers and a step of two
+// columns reads eight new samples for 72 packed operations. Sums run in tap
+// order, the input's first, then the QP plane's, zero in the halo. xt is the
+// zero-padded input by columns. Bound by the fp32 pipe: 590 k multiply-adds
+// are 4.6 k cycles (a thread per pixel and all channels read each weight from
+// shared memory again: 16 k cycles, the load path's rate).
+__device__ __forceinline__ void cnn_layer1(const float* xt, const float2* w1, const float2* b1, float qp_in,
+                                           uint8_t* img, uint16_t* acts, int warp, int lane) {
+  const int c2 = lane & 15, y0 = 4 * warp + 2 * (lane >> 4);
+  uint64_t wx[9], wq[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    wx[k] = ((const uint64_t*)w1)[k * 16 + c2];
+    wq[k] = ((const uint64_t*)w1)[(9 + k) * 16 + c2];
+  }
+  const uint64_t bias = ((const uint64_t*)b1)[c2];
+  const uint64_t q = f2_pack(qp_in, qp_in), q0 = y0 == 0 ? 0ull : q, q3 = y0 == 30 ? 0ull : q;
+  const float* xp = xt + y0;
+  float2 na[2], nb[2];  // rows y0 - 1 .. y0 + 2 of the next two columns
+  auto load = [&](int x) {
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      na[i] = *(const float2*)(xp + (x + i) * kImgW);
+      nb[i] = *(const float2*)(xp + (x + i) * kImgW + 2);
+    }
+  };
+  uint64_t in[4][4];  // columns x - 1 .. x + 2 (a ring), the four rows
+  auto put = [&](int i, uint64_t* v) {
+    v[0] = f2_pack(na[i].x, na[i].x);
+    v[1] = f2_pack(na[i].y, na[i].y);
+    v[2] = f2_pack(nb[i].x, nb[i].x);
+    v[3] = f2_pack(nb[i].y, nb[i].y);
+  };
+  load(0);
+  put(0, in[0]);
+  put(1, in[1]);
+  load(2);
+  put(0, in[2]);
+  put(1, in[3]);
+  uint8_t* dst = img + (c2 >> 2) * kPlane + ((y0 + 1) * kImgW + 1) * 16 + (c2 & 3) * 4;
+  uint32_t* ga = acts ? (uint32_t*)acts + y0 * 32 * 16 + c2 : nullptr;
+  // two columns by two rows at a time: four independent sums
+#pragma unroll 1
+  for (int x0 = 0; x0 < 32; x0 += 4)
+#pragma unroll
+    for (int j = 0; j < 4; j += 2) {
+      const int x = x0 + j;
+      if (x < 30) load(x + 4);
+      uint64_t s[4] = {bias, bias, bias, bias};
+#pragma unroll
+      for (int k = 0; k < 9; k++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) s[i] = f2_fma(wx[k], in[(j + (i & 1) + k % 3) & 3][(i >> 1) + k / 3], s[i]);
+#pragma unroll
+      for (int k = 0; k < 9; k++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const int row = (i >> 1) + k / 3;
+          uint64_t v = row == 0 ? q0 : row == 3 ? q3 : q;
+          if (j == 0 && (i & 1) == 0 && k % 3 == 0 && x0 == 0) v = 0ull;
+          if (j == 2 && (i & 1) == 1 && k % 3 == 2 && x0 == 28) v = 0ull;
+          s[i] = f2_fma(wq[k], v, s[i]);
+        }
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const float2 o = f2_unpack(s[i]);
+        const uint32_t pk = pack_bf2(fmaxf(o.x, 0.0f), fmaxf(o.y, 0.0f));
+        *(uint32_t*)(dst + ((i >> 1) * kImgW + x + (i & 1)) * 16) = pk;
+        if (ga) ga[((i >> 1) * 32 + x + (i & 1)) * 16] = pk;
+      }
+      put(0, in[j & 3]);
+      put(1, in[(j + 1) & 3]);
+    }
+}
+
+// Takes one of the turns of a CTA's two groups, given back by atomicExch. One
+// group at a time is in layer 1 and one at a time issues MMAs: side by side
+// both would take twice as long and then do the next part side by side too,
+// block after block. The turns are only for speed: after some tens of
+// microseconds a group goes on without.
+__device__ __forceinline__ void cnn_take(uint32_t* turn) {
+  for (int i = 0; i < 1024 && atomicCAS(turn, 0u, 1u) != 0u; i++) __nanosleep(32);
+}
+
+// Persistent, one CTA per SM with two groups of 8 warps that work on blocks
+// of their own, independently: while one group's MMAs run, the other adds
+// biases, packs and stores, and the tensor core idles only where both do
+// (one block at a time: MMAs 24 k of a block's 64 k cycles, serial with the
+// rest). Each group's image is written in place, so two images and the
+// weights fill the shared memory as two ping-pong images of one block would;
+// 2 x 256 columns fill the TMEM. The next block's samples are loaded while the
+// current block's layers run. 1980 blocks: 414 us
+// -> 199 us (the tensor core busy for 35 k of the 42 k cycles that two blocks
+// take); without the turns 244 us.
+__global__ void __launch_bounds__(kCnnGroups* kCnnThreads, 1) k_cnn_forward(const __grid_constant__ CnnFwdArgs A) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const int grp = __shfl_sync(0xFFFFFFFFu, (int)threadIdx.x / kCnnThreads, 0);
+  const int t = threadIdx.x % kCnnThreads, warp = __shfl_sync(0xFFFFFFFFu, t >> 5, 0), lane = t & 31;
+  uint8_t* W = smem + kCnnGroups * kImg;
+  float* w1 = (float*)(W + 3 * kPackL);  // [18][32]
+  float* b1 = w1 + 576;
+  float* bias = b1 + 32;                         // [3][32]
+  float* xt = bias + 96 + grp * kCnnGroupF;      // the group's padded input, by columns
+  float* gpart = xt + kXPad;                     // [8 warps][32]
+  float* gap = gpart + 256;                      // [32]
+  float* heads = bias + 96 + kCnnGroups * kCnnGroupF;  // [73][kHeadPitch], then the 73 biases
+  uint64_t* mbars = (uint64_t*)(W + 3 * kPackL + kCnnMisc);
+  uint32_t* tslot = (uint32_t*)(mbars + kCnnGroups);
+  uint32_t* turn = tslot + 1;  // taken: [0] layer 1, [1] the tensor core
+  uint8_t* X = smem + grp * kImg;
+  uint64_t* mbar = mbars + grp;
+
+  // weights, zero images (the halos stay zero), TMEM, barriers
+  constexpr int kAll = kCnnGroups * kCnnThreads;
+  for (int i = threadIdx.x; i < 3 * kPackL / 16; i += kAll) ((uint4*)W)[i] = ((const uint4*)A.pack)[i];
+  for (int i = threadIdx.x; i < kCnnGroups * kImg / 16; i += kAll) ((uint4*)smem)[i] = make_uint4(0, 0, 0, 0);
+  for (int i = threadIdx.x; i < 576; i += kAll) w1[(i % 18) * 32 + i / 18] = A.params[kOffW1 + i];
+  for (int i = threadIdx.x; i < kCnnOut * 32; i += kAll)
+    heads[(i >> 5) * kHeadPitch + (i & 31)] =
+        A.params[(i >> 5) < kCnnModes ? kOffWi + i : kOffWs + i - kCnnModes * 32];
+  if (threadIdx.x < kCnnOut)
+    heads[kCnnOut * kHeadPitch + threadIdx.x] =
+        A.params[threadIdx.x < kCnnModes ? kOffBi + threadIdx.x : kOffBs + threadIdx.x - kCnnModes];
+  for (int i = t; i < kXPad; i += kCnnThreads) xt[i] = 0.0f;
+  if (threadIdx.x < 32) b1[t] = A.params[kOffB1 + t];
+  if (threadIdx.x < 96) bias[t] = A.params[cnn_off_b(2 + t / 32) + t % 32];
+  if (threadIdx.x < 32) {
+    tmem_alloc(tslot, kCnnGroups * 256);
     tmem_relinquish();
   }
   if (t == 0) {
     mbar_init(mbar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    turn[0] = turn[1] = 0;
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tslot;
+  const uint32_t tmem = *tslot + grp * 256;
+  const float inv = 1.0f / (float)A.maxv;
+  const int bar = 1 + grp;
   uint32_t phase = 0;
   bool ok = true;
 
-  for (int blk = blockIdx.x; blk < A.n && ok; blk += gridDim.x) {
-    const uint32_t ux = A.ctu_xy[2 * blk], uy = A.ctu_xy[2 * blk + 1];
-    if (ux > (uint32_t)A.width - 32 || uy > (uint32_t)A.height - 32 || A.width < 32 || A.height < 32) {
+  const int step = kCnnGroups * gridDim.x;
+  int blk = blockIdx.x + grp * gridDim.x;
+  uint16_t px[4];
+  bool inside = blk < A.n && cnn_load_px(A.plane, A.stride, A.width, A.height, A.ctu_xy, blk, t, px);
+  while (blk < A.n) {
+    const int next = blk + step;
+    if (!inside) {
       // a block outside the plane: NaN logits, flagged, nothing read
       if (t < kCnnOut) A.logits[(size_t)blk * kCnnOut + t] = __int_as_float(0x7FC00000);
       if (t == 0) atomicOr(A.status, 2u);
+      blk = next;
+      inside = blk < A.n && cnn_load_px(A.plane, A.stride, A.width, A.height, A.ctu_xy, blk, t, px);
       continue;
     }
-    const int bx = (int)ux, by = (int)uy;
-    const float inv = 1.0f / (float)A.maxv;
-    for (int i = t; i < 1024; i += kCnnThreads)
-      xin[i] = bf2f(f2bf((float)A.plane[(int64_t)(by + (i >> 5)) * A.stride + bx + (i & 31)] * inv));
-    __syncthreads();
-    // layer 1 on the CUDA cores: 4 pixels per thread
-    for (int p = t; p < 1024; p += kCnnThreads) {
-      const int iy = p >> 5, ix = p & 31;
-      float in[9], iq[9];
 #pragma unroll
-      for (int tap = 0; tap < 9; tap++) {
-        const int y = iy + tap / 3 - 1, x = ix + tap % 3 - 1;
-        const bool inside = y >= 0 && y < 32 && x >= 0 && x < 32;
-        in[tap] = inside ? xin[y * 32 + x] : 0.0f;
-        iq[tap] = inside ? A.qp_in : 0.0f;
-      }
-      uint32_t pk[16];
-#pragma unroll
-      for (int c = 0; c < 32; c += 2) {
-        float s0 = b1[c], s1 = b1[c + 1];
-#pragma unroll
-        for (int tap = 0; tap < 9; tap++) {
-          s0 = fmaf(w1[c * 18 + tap], in[tap], s0);
-          s1 = fmaf(w1[(c + 1) * 18 + tap], in[tap], s1);
-        }
-#pragma unroll
-        for (int tap = 0; tap < 9; tap++) {
-          s0 = fmaf(w1[c * 18 + 9 + tap], iq[tap], s0);
-          s1 = fmaf(w1[(c + 1) * 18 + 9 + tap], iq[tap], s1);
-        }
-        pk[c / 2] = (uint32_t)f2bf(fmaxf(s0, 0.0f)) | ((uint32_t)f2bf(fmaxf(s1, 0.0f)) << 16);
-      }
-      const int off = ((iy + 1) * kImgW + ix + 1) * 16;
-#pragma unroll
-      for (int g = 0; g < 4; g++)
-        *(uint4*)(X0 + g * kPlane + off) = make_uint4(pk[4 * g], pk[4 * g + 1], pk[4 * g + 2], pk[4 * g + 3]);
-      if (A.acts) {
-        uint4* dst = (uint4*)(A.acts + (((size_t)blk * 4 + 0) * 1024 + p) * 32);
-#pragma unroll
-        for (int g = 0; g < 4; g++) dst[g] = make_uint4(pk[4 * g], pk[4 * g + 1], pk[4 * g + 2], pk[4 * g + 3]);
-      }
-    }
+    for (int k = 0; k < 4; k++)
+      xt[((t & 31) + 1) * kImgW + (t >> 5) + 8 * k + 1] = bf2f(f2bf((float)px[k] * inv));
+    if (t == 0) cnn_take(turn);
+    cnn_sync(bar);
+    uint16_t* acts = A.acts ? A.acts + (size_t)blk * 4 * 1024 * 32 : nullptr;
+    cnn_layer1(xt, (const float2*)w1, (const float2*)b1, A.qp_in, X, acts, warp, lane);
+    inside = next < A.n && cnn_load_px(A.plane, A.stride, A.width, A.height, A.ctu_xy, next, t, px);
     float acc[32];
 #pragma unroll
     for (int c = 0; c < 32; c++) acc[c] = 0.0f;
-    for (int l = 0; l < 3 && ok; l++) {
-      uint8_t* xi = (l & 1) ? X1 : X0;
-      uint8_t* xo = (l & 1) ? X0 : X1;
+#pragma unroll 1
+    for (int l = 0; l < 3; l++) {
       fence_async_smem();
       tc_fence_before();
-      __syncthreads();
+      cnn_sync(bar);
       tc_fence_after();
-      if (t == 0) cnn_issue_layer(tmem, smem_u32(xi), smem_u32(W) + l * kPackL, mbar);
-      ok = __syncthreads_and(mbar_wait(mbar, phase, 1u << 26));
+      if (warp == 0 && elect_one()) {
+        if (l == 0) atomicExch(turn, 0u);
+        cnn_take(turn + 1);
+        cnn_issue_layer(tmem, smem_u32(X), smem_u32(W) + l * kPackL, mbar);
+        atomicExch(turn + 1, 0u);
+      }
+      __syncwarp();
+      ok = cnn_sync_and(bar, mbar_wait(mbar, phase, 1u << 26));
       phase ^= 1;
       tc_fence_after();
       if (!ok) break;
       const int q = warp & 3;
+#pragma unroll 1
       for (int k = 0; k < 4; k++) {
         const int tile = (warp >> 2) + 2 * k;
         const int m = 32 * q + lane, j = m >> 3, r = m & 7;
         const int iy = 16 * (tile >> 2) + j, ix = 8 * (tile & 3) + r;
         float v[32];
-        tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + tile * 32, v);
-        tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + tile * 32 + 16, v + 16);
+        tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + tile * 32, v);
 #pragma unroll
-        for (int c = 0; c < 32; c++) v[c] = fmaxf(v[c] + bias[l * 32 + c], 0.0f);
-        if (l < 2 || A.acts) {
-          uint32_t pk[16];
+        for (int c = 0; c < 32; c += 4) {
+          const float4 b = *(const float4*)(bias + l * 32 + c);
+          v[c] = fmaxf(v[c] + b.x, 0.0f);
+          v[c + 1] = fmaxf(v[c + 1] + b.y, 0.0f);
+          v[c + 2] = fmaxf(v[c + 2] + b.z, 0.0f);
+          v[c + 3] = fmaxf(v[c + 3] + b.w, 0.0f);
+        }
+        if (l < 2 || acts) {
+          const int off = ((iy + 1) * kImgW + ix + 1) * 16;
+          uint4* dst = acts ? (uint4*)(acts + ((size_t)(l + 1) * 1024 + iy * 32 + ix) * 32) : nullptr;
 #pragma unroll
-          for (int c = 0; c < 32; c += 2) pk[c / 2] = (uint32_t)f2bf(v[c]) | ((uint32_t)f2bf(v[c + 1]) << 16);
-          if (l < 2) {
-            const int off = ((iy + 1) * kImgW + ix + 1) * 16;
-#pragma unroll
-            for (int g = 0; g < 4; g++)
-              *(uint4*)(xo + g * kPlane + off) = make_uint4(pk[4 * g], pk[4 * g + 1], pk[4 * g + 2], pk[4 * g + 3]);
-          }
-          if (A.acts) {
-            uint4* dst = (uint4*)(A.acts + (((size_t)blk * 4 + l + 1) * 1024 + iy * 32 + ix) * 32);
-#pragma unroll
-            for (int g = 0; g < 4; g++) dst[g] = make_uint4(pk[4 * g], pk[4 * g + 1], pk[4 * g + 2], pk[4 * g + 3]);
+          for (int g = 0; g < 4; g++) {
+            const uint4 pk = make_uint4(pack_bf2(v[8 * g], v[8 * g + 1]), pack_bf2(v[8 * g + 2], v[8 * g + 3]),
+                                        pack_bf2(v[8 * g + 4], v[8 * g + 5]), pack_bf2(v[8 * g + 6], v[8 * g + 7]));
+            if (l < 2) *(uint4*)(X + g * kPlane + off) = pk;
+            if (dst) dst[g] = pk;
           }
         }
         if (l == 2) {
@@ -232,33 +398,28 @@ __global__ void __launch_bounds__(kCnnThreads, 1) k_cnn_forward(const __grid_con
     }
     if (!ok) break;
     // global average: the warp's 128 pixels, then the 8 warps
-#pragma unroll
-    for (int c = 0; c < 32; c++) {
-      float s = acc[c];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-      if (lane == 0) gpart[warp * 32 + c] = s;
-    }
+    gpart[warp * 32 + lane] = warp_sum32(acc, lane);
     tc_fence_before();
-    __syncthreads();
+    cnn_sync(bar);
     if (t < 32) {
       float s = 0.0f;
       for (int w = 0; w < 8; w++) s += gpart[w * 32 + t];
       gap[t] = s * (1.0f / 1024.0f);
       if (A.gap_out) A.gap_out[(size_t)blk * 32 + t] = gap[t];
     }
-    __syncthreads();
+    cnn_sync(bar);
     if (t < kCnnOut) {
-      const float* Wh = t < kCnnModes ? A.params + kOffWi + t * 32 : A.params + kOffWs + (t - kCnnModes) * 32;
-      float s = t < kCnnModes ? A.params[kOffBi + t] : A.params[kOffBs + t - kCnnModes];
+      const float* Wh = heads + t * kHeadPitch;
+      float s = heads[kCnnOut * kHeadPitch + t];
       for (int c = 0; c < 32; c++) s = fmaf(Wh[c], gap[c], s);
       A.logits[(size_t)blk * kCnnOut + t] = s;
     }
+    blk = next;
   }
   if (!ok && t == 0) atomicOr(A.status, 1u);
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, 256);
+  if (threadIdx.x < 32) tmem_dealloc(*tslot, kCnnGroups * 256);
 }
 
 }  // namespace vvcg
@@ -299,7 +460,6 @@ struct CnnBwdArgs {
   float inv_batch;
   uint32_t* status;
 };
-constexpr int kXPad = 34 * 34;  // the input zero-padded by one pixel
 constexpr int kCnnBwdMisc = (2 * kXPad + 32 + 32 * 8 + 96) * 4;
 // M = 64, N = 32, both operands MN-major
 constexpr uint32_t kCnnIdescW = umma_idesc_bf16(64, 32) | (1u << 15) | (1u << 16);

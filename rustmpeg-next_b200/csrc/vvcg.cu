@@ -1748,7 +1748,7 @@ extern "C" vvcg_status vvcg_cnn_forward_dev(vvcg_ctx* ctx, const uint16_t* plane
   CnnFwdArgs A{plane, (int64_t)stride, (int32_t)width, (int32_t)height, (1 << bit_depth) - 1, (int32_t)num_blocks,
                cnn_qp_input(qp), ctu_xy, params, (const uint16_t*)ctx->d_cnn_pack.p, logits, gap, acts, status};
   const uint32_t grid = std::min<uint32_t>(num_blocks, (uint32_t)ctx->num_sms);
-  k_cnn_forward<<<grid, kCnnThreads, kCnnSmem, ctx->stream>>>(A);
+  k_cnn_forward<<<grid, kCnnGroups * kCnnThreads, kCnnSmem, ctx->stream>>>(A);
   CK(cudaGetLastError(), "cnn launch");
   ctx->launches += 2;
   return VVCG_OK;
@@ -1819,7 +1819,7 @@ static vvcg_status cnn_train_step(vvcg_ctx* ctx, const uint16_t* plane, uint64_t
   CnnFwdArgs F{plane, (int64_t)stride, (int32_t)width, (int32_t)height, (1 << bit_depth) - 1, (int32_t)num_blocks,
                cnn_qp_input(qp), ctu_xy, params, (const uint16_t*)ctx->d_cnn_pack.p, (float*)ctx->d_cnn_logits.p,
                (float*)ctx->d_cnn_gap.p, (uint16_t*)ctx->d_cnn_acts.p, status};
-  k_cnn_forward<<<grid, kCnnThreads, kCnnSmem, ctx->stream>>>(F);
+  k_cnn_forward<<<grid, kCnnGroups * kCnnThreads, kCnnSmem, ctx->stream>>>(F);
   CK(cudaGetLastError(), "cnn forward launch");
   CnnBwdArgs B{plane, (int64_t)stride, (int32_t)width, (int32_t)height, (1 << bit_depth) - 1, (int32_t)num_blocks,
                cnn_qp_input(qp), ctu_xy, labels, params, soft, (const uint16_t*)ctx->d_cnn_packT.p,
