@@ -77,18 +77,21 @@ __device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
-// Sums v[c] over the warp for 32 channels c, into lane c: each step halves
-// the channels a lane carries (31 shuffles instead of 160; the additions pair
-// the same lanes, at distances 16, 8, 4, 2, 1, as a butterfly per channel).
-__device__ __forceinline__ float warp_sum32(float* v, int lane) {
+// Sums v[c] over the warp for kN channels c, into the lanes of number
+// c * 32 / kN on: each step halves the channels that a lane carries (31
+// shuffles for 32 channels instead of 160; the additions pair the same lanes,
+// at distances 16, 8, 4, 2, 1, as a butterfly per channel).
+template <int kN>
+__device__ __forceinline__ float warp_sum(float* v, int lane) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+  for (int o = 16, n = kN / 2; o > 0; o >>= 1, n >>= 1) {
     const bool up = lane & o;
 #pragma unroll
-    for (int c = 0; c < o; c++) {
-      const float send = up ? v[c] : v[c + o], keep = up ? v[c + o] : v[c];
+    for (int c = 0; c < n; c++) {
+      const float send = up ? v[c] : v[c + n], keep = up ? v[c + n] : v[c];
       v[c] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, o);
     }
+    if (n == 0) v[0] += __shfl_xor_sync(0xFFFFFFFFu, v[0], o);
   }
   return v[0];
 }
@@ -398,7 +401,7 @@ __global__ void __launch_bounds__(kCnnGroups* kCnnThreads, 1) k_cnn_forward(cons
     }
     if (!ok) break;
     // global average: the warp's 128 pixels, then the 8 warps
-    gpart[warp * 32 + lane] = warp_sum32(acc, lane);
+    gpart[warp * 32 + lane] = warp_sum<32>(acc, lane);
     tc_fence_before();
     cnn_sync(bar);
     if (t < 32) {
@@ -428,8 +431,8 @@ namespace vvcg {
 
 // ---------------------------------------------------------------- backward --
 //
-// One CTA per block (persistent). From the forward's activations a1..a4,
-// gap and logits: the head gradients, then per layer l = 4, 3, 2 the
+// One CTA of 16 warps per block (persistent). From the forward's activations
+// a1..a4, gap and logits: the head gradients, then per layer l = 4, 3, 2 the
 // gradient dZ_l (w.r.t. the layer's pre-activation) held as a bf16 image:
 //  * its input gradient dA_{l-1} = conv(dZ_l, flipped W_l) is 144 tcgen05
 //    MMAs exactly as in the forward pass (the taps of the transposed
@@ -441,8 +444,17 @@ namespace vvcg {
 //  * the epilogue masks dA_{l-1} by a_{l-1} > 0 into dZ_{l-1}, in place of
 //    a_{l-1}.
 // Layer 1's weight gradient uses the bf16 input. Gradients and the loss
-// accumulate in the CTA's own slice of `partial` (no atomics); a second
-// kernel sums the slices.
+// accumulate in the CTA's own slice of `partial` (no atomics), laid out as
+// the threads hold them; a second kernel sums the slices into the parameter
+// order.
+//
+// The two halves of the warps take 16 channels each of the same pixels, so
+// every sum keeps one order whatever the number of warps. Beside the MMAs:
+// the activations come by cp.async, the next layer's (or block's) into the
+// buffer that the layer has done with, during its epilogue; a layer's weight
+// gradient is read out of TMEM while the next input gradient's MMAs run.
+// 1024 blocks: 958 -> 447 us, the 432 + 1728 MMAs of a block 62 k of 106 k cycles
+// at the rate of their operand reads.
 struct CnnBwdArgs {
   const uint16_t* plane;
   int64_t stride;
@@ -460,7 +472,14 @@ struct CnnBwdArgs {
   float inv_batch;
   uint32_t* status;
 };
-constexpr int kCnnBwdMisc = (2 * kXPad + 32 + 32 * 8 + 96) * 4;
+constexpr int kCnnBwdThreads = 512;
+constexpr int kCnnBwdRed = 8 * 32 * 18;  // layer 1's partial weight gradients
+constexpr int kCnnBwdMisc = (kXPad + 32 + 32 * 8 + 96 + kCnnBwdRed) * 4;
+// A CTA's slice of the partial sums, in floats: per layer 2..4, tap pair and
+// column the 64 values of one TMEM column (cnn_slice_w), then W1 and b1, the
+// three biases, the heads and the loss.
+constexpr int kSlW1 = 3 * 5 * 32 * 64, kSlB = kSlW1 + 608, kSlHeads = kSlB + 96;
+constexpr int kSlLoss = kSlHeads + kCnnParams - kOffWi, kCnnSlice = (kSlLoss + 1 + 3) / 4 * 4;
 // M = 64, N = 32, both operands MN-major
 constexpr uint32_t kCnnIdescW = umma_idesc_bf16(64, 32) | (1u << 15) | (1u << 16);
 constexpr int kCnnBwdCols = 512;  // dA_{l-1}: columns 0..255; dW_l: 256..415
@@ -478,56 +497,100 @@ constexpr int kCnnBwdCols = 512;  // dA_{l-1}: columns 0..255; dW_l: 256..415
 // 16 (t & 1) + {0..15, 32..47} of columns (t >> 1) * 32 + 0..31 (two M = 64
 // accumulators share columns in the two half sub-partitions).
 __device__ __forceinline__ void cnn_issue_dw(uint32_t tmem, uint32_t lo, uint32_t hi, bool lo_tap) {
-  // the start address is the descriptor's low field in 16-byte units (one
-  // pixel): every operand is a base descriptor plus a pixel offset
-  const uint64_t da0 = umma_desc(lo, 128, kPlane), db0 = umma_desc(hi, 128, kPlane);
+  // Bound by the operands' shared-memory reads, 2 KB of L and 1 KB of H per MMA
+  // at 128 B per cycle (24 cycles, as measured).
+  constexpr uint64_t kD = umma_desc(0, 128, kPlane);
+  const uint32_t a0 = (uint32_t)kD + (lo >> 4), b0 = (uint32_t)kD + (hi >> 4), ma = lo_tap ? 0xFFFFFFFFu : 0u;
+#pragma unroll 1
   for (int y = 0; y < 32; y++)
+#pragma unroll
     for (int h = 0; h < 2; h++) {
-      const int base = (y + 1) * kImgW + 1 + 16 * h;
+      const uint32_t base = (y + 1) * kImgW + 1 + 16 * h;
 #pragma unroll
       for (int tap = 0; tap < 9; tap++) {
-        const int sh = (tap / 3 - 1) * kImgW + tap % 3 - 1;
+        const uint32_t sh = (uint32_t)((tap / 3 - 1) * kImgW + tap % 3 - 1);
         umma_bf16(tmem + ((uint32_t)(16 * (tap & 1)) << 16) + (tap >> 1) * 32,
-                  da0 + (uint64_t)(base + (lo_tap ? sh : 0)), db0 + (uint64_t)(base + (lo_tap ? 0 : sh)),
+                  (kD >> 32 << 32) | (a0 + base + (sh & ma)), (kD >> 32 << 32) | (b0 + base + (sh & ~ma)),
                   kCnnIdescW, (y | h) != 0);
       }
     }
 }
-constexpr int kCnnBwdSmem = 2 * kImg + kPackL + kCnnBwdMisc + 64;
+constexpr int kCnnBwdSmem = 2 * kImg + 3 * kPackL + kCnnBwdMisc + 64;
+static_assert(kCnnBwdSmem <= 227 * 1024, "backward shared memory");
 
-// Loads activation image `layer` (0..3) of block blk from global into an
-// image buffer (interior only; the halo stays zero).
+// Starts the copy of activation image `layer` (0..3) of block blk from global
+// into an image buffer (interior only; the halo stays zero) as one cp.async
+// group of every thread.
 __device__ __forceinline__ void cnn_load_act(uint8_t* img, const uint16_t* acts, int blk, int layer) {
   const uint4* src = (const uint4*)(acts + ((size_t)blk * 4 + layer) * 1024 * 32);
-  for (int i0 = threadIdx.x; i0 < 1024 * 4; i0 += 4 * kCnnThreads) {
-    uint4 v[4];  // four loads in flight before the stores
 #pragma unroll
-    for (int k = 0; k < 4; k++) v[k] = src[i0 + k * kCnnThreads];
+  for (int k = 0; k < 1024 * 4 / kCnnBwdThreads; k++) {
+    const int i = threadIdx.x + k * kCnnBwdThreads, p = i >> 2, g = i & 3;
+    const uint32_t dst = smem_u32(img + g * kPlane + (((p >> 5) + 1) * kImgW + (p & 31) + 1) * 16);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src + i) : "memory");
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int kPending>
+__device__ __forceinline__ void cnn_load_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
+}
+
+// The first block from blk on (in steps of the grid) that lies inside the
+// plane with labels in range; flags the skipped ones.
+__device__ __forceinline__ int cnn_next_block(const CnnBwdArgs& A, int blk) {
+  for (; blk < A.n; blk += gridDim.x) {
+    const uint32_t ux = A.ctu_xy[2 * blk], uy = A.ctu_xy[2 * blk + 1];
+    if (!(ux > (uint32_t)A.width - 32 || uy > (uint32_t)A.height - 32 || A.width < 32 || A.height < 32 ||
+          A.labels[2 * blk] >= kCnnModes || A.labels[2 * blk + 1] >= kCnnSplits))
+      break;
+    if (threadIdx.x == 0) atomicOr(A.status, 2u);
+  }
+  return blk;
+}
+
+// Adds the weight gradient in TMEM to the slice of layer li: lane quarters 0
+// and 1 hold rows 0..31 (the channels of the image at P), a lane tap
+// 2 g + lane / 16 of row 16 q + lane % 16, a column the other image's channel.
+__device__ __forceinline__ void cnn_drain_dw(float* part, uint32_t tmem, int li, int warp, int lane) {
+  const int q = warp & 3;
+  if (q >= 2) return;
+#pragma unroll 1
+  for (int u = warp >> 2; u < 10; u += kCnnBwdThreads / 128) {
+    const int g = u >> 1;
+    float v[16], o[16];
+    tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + u * 16, v);
+    if (2 * g + (lane >> 4) < 9) {  // the loads first, then the stores
+      float* d = part + ((li * 5 + g) * 32 + (u & 1) * 16) * 64 + q * 32 + lane;
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int i = i0 + k * kCnnThreads, p = i >> 2, g = i & 3;
-      *(uint4*)(img + g * kPlane + (((p >> 5) + 1) * kImgW + (p & 31) + 1) * 16) = v[k];
+      for (int n = 0; n < 16; n++) o[n] = d[n * 64];
+#pragma unroll
+      for (int n = 0; n < 16; n++) d[n * 64] = o[n] + v[n];
     }
   }
 }
 
-__global__ void __launch_bounds__(kCnnThreads, 1) k_cnn_backward(const __grid_constant__ CnnBwdArgs A) {
+__global__ void __launch_bounds__(kCnnBwdThreads, 1) k_cnn_backward(const __grid_constant__ CnnBwdArgs A) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* P = smem;
   uint8_t* Q = smem + kImg;
   uint8_t* Wt = smem + 2 * kImg;
-  // (bf16-rounded normalised input, 1) inside the block, (0, 0) in the halo
-  float2* xpad = (float2*)(Wt + kPackL);
+  // (bf16 normalised input, bf16 1) inside the block, (0, 0) in the halo
+  uint32_t* xpad = (uint32_t*)(Wt + 3 * kPackL);
   float* dgap = (float*)(xpad + kXPad);
   float* dbp = dgap + 32;   // [8 warps][32] bias-gradient partials
   float* dlog = dbp + 256;  // [73] logit gradients (+ pad)
-  uint64_t* mbar = (uint64_t*)(dlog + 96);
+  float* red = dlog + 96;   // [8 row groups][32 channels][18]
+  uint64_t* mbar = (uint64_t*)(Wt + 3 * kPackL + kCnnBwdMisc);
   uint32_t* tslot = (uint32_t*)(mbar + 1);
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  float* part = A.partial + (size_t)blockIdx.x * (kCnnParams + 1);
-  for (int i = t; i < kCnnParams + 1; i += kCnnThreads) part[i] = 0.0f;
-  for (int i = t; i < 2 * kImg / 16; i += kCnnThreads) ((uint4*)P)[i] = make_uint4(0, 0, 0, 0);
-  for (int i = t; i < kXPad; i += kCnnThreads) xpad[i] = make_float2(0.0f, 0.0f);
+  const int t = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, t >> 5, 0), lane = t & 31;
+  const int hw = warp >> 3, w8 = warp & 7;  // channel half, warp within it
+  float* part = A.partial + (size_t)blockIdx.x * kCnnSlice;
+  int blk = cnn_next_block(A, blockIdx.x);
+  for (int i = t; i < kCnnSlice / 4; i += kCnnBwdThreads) ((float4*)part)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  for (int i = t; i < 2 * kImg / 16; i += kCnnBwdThreads) ((uint4*)P)[i] = make_uint4(0, 0, 0, 0);
+  for (int i = t; i < 3 * kPackL / 16; i += kCnnBwdThreads) ((uint4*)Wt)[i] = ((const uint4*)A.packT)[i];
+  for (int i = t; i < kXPad; i += kCnnBwdThreads) xpad[i] = 0;
   if (warp == 0) {
     tmem_alloc(tslot, kCnnBwdCols);
     tmem_relinquish();
@@ -542,14 +605,13 @@ __global__ void __launch_bounds__(kCnnThreads, 1) k_cnn_backward(const __grid_co
   const uint32_t tmem = *tslot;
   uint32_t phase = 0;
   bool ok = true;
+  int pending = -1;  // the layer (minus 2) whose weight gradient is in TMEM
 
-  for (int blk = blockIdx.x; blk < A.n && ok; blk += gridDim.x) {
-    const uint32_t ux = A.ctu_xy[2 * blk], uy = A.ctu_xy[2 * blk + 1];
-    if (ux > (uint32_t)A.width - 32 || uy > (uint32_t)A.height - 32 || A.width < 32 || A.height < 32 ||
-        A.labels[2 * blk] >= kCnnModes || A.labels[2 * blk + 1] >= kCnnSplits) {
-      if (t == 0) atomicOr(A.status, 2u);  // skipped: outside the plane or a label out of range
-      continue;
-    }
+  if (blk < A.n) cnn_load_act(P, A.acts, blk, 3);
+  while (blk < A.n) {
+    cnn_load_act(Q, A.acts, blk, 2);
+    const int bx = (int)A.ctu_xy[2 * blk], by = (int)A.ctu_xy[2 * blk + 1];
+    float hwt[kCnnOut];  // warp 2: its channel's head weights, loaded beside the softmax
     // heads: softmax cross-entropy of both heads, mean over the batch
     if (warp == 0 || warp == 1) {
       const float* lg = A.logits + (size_t)blk * kCnnOut;
@@ -574,252 +636,251 @@ __global__ void __launch_bounds__(kCnnThreads, 1) k_cnn_backward(const __grid_co
       if (tg)
         for (int o = 16; o > 0; o >>= 1) ce += __shfl_xor_sync(0xFFFFFFFFu, ce, o);
       if (lane == 0) dlog[kCnnOut + warp] = (tg ? ce : (logf(se) + mx - lg[base + label])) * A.inv_batch;
+    } else if (warp == 2) {
+#pragma unroll
+      for (int j = 0; j < kCnnOut; j++)
+        hwt[j] = A.params[(j < kCnnModes ? kOffWi : kOffWs - kCnnModes * 32) + j * 32 + lane];
+    } else if (warp >= 8) {
+      const float inv = 1.0f / (float)A.maxv;
+      uint16_t pv[4];  // the loads first, then the stores
+#pragma unroll
+      for (int u = 0; u < 4; u++) pv[u] = A.plane[(int64_t)(by + w8 + 8 * u) * A.stride + bx + lane];
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        xpad[(w8 + 8 * u + 1) * 34 + lane + 1] = (uint32_t)f2bf((float)pv[u] * inv) | 0x3F800000u;
     }
     __syncthreads();
     // the two heads' losses, added in a fixed order (training is deterministic)
-    if (t == 0) part[kCnnParams] += dlog[kCnnOut] + dlog[kCnnOut + 1];
-    const float inv = 1.0f / (float)A.maxv;
-    const int bx = (int)ux, by = (int)uy;
-    {
-      uint16_t pv[1024 / kCnnThreads];  // the loads first, then the stores
-#pragma unroll
-      for (int u = 0; u < 1024 / kCnnThreads; u++) {
-        const int i = t + u * kCnnThreads;
-        pv[u] = A.plane[(int64_t)(by + (i >> 5)) * A.stride + bx + (i & 31)];
-      }
-#pragma unroll
-      for (int u = 0; u < 1024 / kCnnThreads; u++) {
-        const int i = t + u * kCnnThreads;
-        xpad[((i >> 5) + 1) * 34 + (i & 31) + 1] = make_float2(bf2f(f2bf((float)pv[u] * inv)), 1.0f);
-      }
-    }
-    __syncthreads();
-    const float* gp = A.gap + (size_t)blk * 32;
-    if (t < 32) {
+    if (t == 0) part[kSlLoss] += dlog[kCnnOut] + dlog[kCnnOut + 1];
+    if (warp == 2) {
       float s = 0.0f;
-      for (int j = 0; j < kCnnModes; j++) s = fmaf(A.params[kOffWi + j * 32 + t], dlog[j], s);
-      for (int j = 0; j < kCnnSplits; j++) s = fmaf(A.params[kOffWs + j * 32 + t], dlog[kCnnModes + j], s);
-      dgap[t] = s;
-    }
-    {
-      constexpr int kR = (kCnnOut * 32 + kCnnThreads - 1) / kCnnThreads;
-      float o[kR];  // the loads first, then the stores
+#pragma unroll
+      for (int j = 0; j < kCnnOut; j++) s = fmaf(hwt[j], dlog[j], s);
+      dgap[lane] = s;
+    } else if (warp > 2) {
+      const float* gp = A.gap + (size_t)blk * 32;
+      const float gv = gp[lane];
+      constexpr int kR = (kCnnOut + 12) / 13;  // rows of the head weights per warp
+      float* ph = part + kSlHeads;             // both heads' rows, 67 biases between them
+      float o[kR];                             // the loads first, then the stores
 #pragma unroll
       for (int k = 0; k < kR; k++) {
-        const int i = t + k * kCnnThreads;
-        if (i < kCnnOut * 32) o[k] = part[((i >> 5) < kCnnModes ? kOffWi : kOffWs - kCnnModes * 32) + i];
+        const int j = warp - 3 + 13 * k;
+        if (j < kCnnOut) o[k] = ph[(j < kCnnModes ? 0 : kCnnModes) + j * 32 + lane];
       }
 #pragma unroll
       for (int k = 0; k < kR; k++) {
-        const int i = t + k * kCnnThreads, j = i >> 5;
-        if (i < kCnnOut * 32) part[(j < kCnnModes ? kOffWi : kOffWs - kCnnModes * 32) + i] = o[k] + dlog[j] * gp[i & 31];
+        const int j = warp - 3 + 13 * k;
+        if (j < kCnnOut) ph[(j < kCnnModes ? 0 : kCnnModes) + j * 32 + lane] = o[k] + dlog[j] * gv;
       }
+    } else {  // the head biases
+      for (int j = t; j < kCnnOut; j += 64)
+        part[kSlHeads + (j < kCnnModes ? kOffBi - kOffWi + j : kOffBs - kOffWi + j - kCnnModes)] += dlog[j];
     }
-    if (t < kCnnOut) part[t < kCnnModes ? kOffBi + t : kOffBs + t - kCnnModes] += dlog[t];
+    cnn_load_wait<1>();
     __syncthreads();
-    // dZ4 into P (a4 > 0 passes dgap / 1024), a3 into Q
+    // dZ4 in place of a4 (a4 > 0 passes dgap / 1024): four channels of every
+    // 64th pixel, a3 on its way into Q
     {
-      const uint4* a4 = (const uint4*)(A.acts + ((size_t)blk * 4 + 3) * 1024 * 32);
-      float dbs[8];
-      for (int k = 0; k < 8; k++) dbs[k] = 0.0f;
-      for (int i0 = t; i0 < 1024 * 4; i0 += 8 * kCnnThreads) {
-        uint4 avs[8];  // eight loads in flight
+      const int t8 = t & 255, g = t8 & 3;
+      const float* dg = dgap + g * 8 + hw * 4;
+      const float d[4] = {dg[0] * (1.0f / 1024.0f), dg[1] * (1.0f / 1024.0f), dg[2] * (1.0f / 1024.0f),
+                          dg[3] * (1.0f / 1024.0f)};
+      float dbs[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 4
+      for (int u = 0; u < 16; u++) {
+        const int p = (t8 >> 2) + 64 * u;
+        uint2* a = (uint2*)(P + g * kPlane + (((p >> 5) + 1) * kImgW + (p & 31) + 1) * 16 + hw * 8);
+        const uint2 av = *a;
+        const uint32_t aw[2] = {av.x, av.y};
+        uint32_t o[2];
 #pragma unroll
-        for (int u = 0; u < 8; u++) avs[u] = a4[i0 + u * kCnnThreads];
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-          const int i = i0 + u * kCnnThreads, p = i >> 2, g = i & 3;  // g is fixed per thread (stride 256)
-          const uint32_t aw[4] = {avs[u].x, avs[u].y, avs[u].z, avs[u].w};
-          uint32_t o[4];
-          for (int k = 0; k < 4; k++) {
-            const float d0 = (aw[k] & 0xFFFFu) && !(aw[k] & 0x8000u) ? dgap[g * 8 + 2 * k] * (1.0f / 1024.0f) : 0.0f;
-            const float d1 =
-                (aw[k] >> 16) && !(aw[k] & 0x80000000u) ? dgap[g * 8 + 2 * k + 1] * (1.0f / 1024.0f) : 0.0f;
-            dbs[2 * k] += d0;
-            dbs[2 * k + 1] += d1;
-            o[k] = (uint32_t)f2bf(d0) | ((uint32_t)f2bf(d1) << 16);
-          }
-          *(uint4*)(P + g * kPlane + (((p >> 5) + 1) * kImgW + (p & 31) + 1) * 16) =
-              make_uint4(o[0], o[1], o[2], o[3]);
+        for (int k = 0; k < 2; k++) {
+          const float d0 = (aw[k] & 0xFFFFu) && !(aw[k] & 0x8000u) ? d[2 * k] : 0.0f;
+          const float d1 = (aw[k] >> 16) && !(aw[k] & 0x80000000u) ? d[2 * k + 1] : 0.0f;
+          dbs[2 * k] += d0;
+          dbs[2 * k + 1] += d1;
+          o[k] = pack_bf2(d0, d1);
         }
+        *a = make_uint2(o[0], o[1]);
       }
       // the 64 threads with the same g hold that plane's sums: reduced over
       // the warp's lanes of equal g, then over the warps in a fixed order
-      for (int k = 0; k < 8; k++) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
         float s2 = dbs[k];
+#pragma unroll
         for (int o2 = 4; o2 < 32; o2 <<= 1) s2 += __shfl_xor_sync(0xFFFFFFFFu, s2, o2);
-        if (lane < 4) dbp[warp * 32 + lane * 8 + k] = s2;
-      }
-      __syncthreads();
-      if (t < 32) {
-        float s2 = 0.0f;
-        for (int w2 = 0; w2 < 8; w2++) s2 += dbp[w2 * 32 + t];
-        part[cnn_off_b(4) + t] += s2;
+        if (lane < 4) dbp[w8 * 32 + lane * 8 + hw * 4 + k] = s2;
       }
     }
-    cnn_load_act(Q, A.acts, blk, 2);
+    const int next = cnn_next_block(A, blk + gridDim.x);
     uint8_t* dz = P;  // dZ_l
     uint8_t* act = Q; // a_{l-1}, becomes dZ_{l-1}
-    for (int layer = 4; layer >= 2 && ok; layer--) {
+#pragma unroll 1
+    for (int layer = 4; layer >= 2; layer--) {
       const int li = layer - 2;
-      {
-        constexpr int kN = kPackL / 16, kU = (kN + kCnnThreads - 1) / kCnnThreads;
-        const uint4* src = (const uint4*)(A.packT + (size_t)li * (kPackL / 2));
-        uint4 wv[kU];  // the loads first, then the stores
-#pragma unroll
-        for (int u = 0; u < kU; u++)
-          if (t + u * kCnnThreads < kN) wv[u] = src[t + u * kCnnThreads];
-#pragma unroll
-        for (int u = 0; u < kU; u++)
-          if (t + u * kCnnThreads < kN) ((uint4*)Wt)[t + u * kCnnThreads] = wv[u];
-      }
+      cnn_load_wait<0>();
       fence_async_smem();
       tc_fence_before();
       __syncthreads();
       tc_fence_after();
-      if (t == 0) {
-        cnn_issue_layer(tmem, smem_u32(dz), smem_u32(Wt), mbar, false);
-        cnn_issue_dw(tmem + 256, smem_u32(P), smem_u32(Q), act == P);
-        umma_commit(mbar);
+      if (warp == 2) {
+        if (elect_one()) cnn_issue_layer(tmem, smem_u32(dz), smem_u32(Wt) + li * kPackL, mbar, false);
+        __syncwarp();
+      } else if (pending >= 0) {
+        cnn_drain_dw(part, tmem + 256, pending, warp, lane);
+      }
+      if (warp == 3) {  // the bias gradient of this layer
+        float s = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 8; w++) s += dbp[w * 32 + lane];
+        part[kSlB + li * 32 + lane] += s;
+      }
+      tc_fence_before();
+      __syncthreads();
+      tc_fence_after();
+      if (warp == 2) {
+        if (elect_one()) {
+          cnn_issue_dw(tmem + 256, smem_u32(P), smem_u32(Q), act == P);
+          umma_commit(mbar);
+        }
+        __syncwarp();
       }
       ok = __syncthreads_and(mbar_wait(mbar, phase, 1u << 26));
       phase ^= 1;
       tc_fence_after();
       if (!ok) break;
-      // weight gradient out of TMEM: warps of lane quarters 0 and 1 hold
-      // rows 0..31 (the channels of the image at P); a thread takes tap
-      // 2g + lane / 16 of row 16 q + lane % 16 and its 32 columns (the other
-      // image's channels)
-      if ((warp & 3) < 2) {
-        float* gw = part + cnn_off_w(layer);
-        const bool rows_co = dz == P;
-        const int r = 16 * (warp & 3) + (lane & 15);
-        for (int g = warp < 4 ? 0 : 3; g < (warp < 4 ? 3 : 5); g++) {
-          const int tp = 2 * g + (lane >> 4);
-          const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 256 + g * 32;
-          float v[32];
-          tmem_ld16(ta, v);
-          tmem_ld16(ta + 16, v + 16);
-          if (tp < 9) {  // the 32 loads first, then the 32 stores (one round trip, not 32)
-            float* g0 = gw + (rows_co ? r * kCnnCh * 9 : r * 9) + tp;
-            const int st = rows_co ? 9 : kCnnCh * 9;
-            float o[32];
-#pragma unroll
-            for (int n = 0; n < 32; n++) o[n] = g0[n * st];
-#pragma unroll
-            for (int n = 0; n < 32; n++) g0[n * st] = o[n] + v[n];
-          }
-        }
-      }
+      pending = li;
+      // the old dZ_l buffer takes a_{l-2}, or the next block's a4
+      if (layer > 2)
+        cnn_load_act(dz, A.acts, blk, layer - 3);
+      else if (next < A.n)
+        cnn_load_act(dz, A.acts, next, 3);
       // epilogue: dZ_{l-1} = dA_{l-1} where a_{l-1} > 0, in place of a_{l-1}
-      float dbs[32];
-      for (int c = 0; c < 32; c++) dbs[c] = 0.0f;
+      float dbs[16];
+#pragma unroll
+      for (int c = 0; c < 16; c++) dbs[c] = 0.0f;
       const int q = warp & 3;
+#pragma unroll 2
       for (int k = 0; k < 4; k++) {
-        const int tile = (warp >> 2) + 2 * k;
+        const int tile = (w8 >> 2) + 2 * k;
         const int m = 32 * q + lane, j = m >> 3, r = m & 7;
         const int iy = 16 * (tile >> 2) + j, ix = 8 * (tile & 3) + r;
-        float v[32];
-        tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + tile * 32, v);
-        tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + tile * 32 + 16, v + 16);
-        const int off = ((iy + 1) * kImgW + ix + 1) * 16;
-        for (int g = 0; g < 4; g++) {
-          uint4 av = *(const uint4*)(act + g * kPlane + off);
-          uint32_t aw[4] = {av.x, av.y, av.z, av.w}, o[4];
+        float v[16];
+        tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + tile * 32 + hw * 16, v);
+        uint8_t* ap = act + 2 * hw * kPlane + ((iy + 1) * kImgW + ix + 1) * 16;
+#pragma unroll
+        for (int g = 0; g < 2; g++) {
+          const uint4 av = *(const uint4*)(ap + g * kPlane);
+          const uint32_t aw[4] = {av.x, av.y, av.z, av.w};
+          uint32_t o[4];
+#pragma unroll
           for (int k2 = 0; k2 < 4; k2++) {
             const int c = g * 8 + 2 * k2;
             const float d0 = ((aw[k2] & 0xFFFFu) && !(aw[k2] & 0x8000u)) ? v[c] : 0.0f;
             const float d1 = ((aw[k2] >> 16) && !(aw[k2] & 0x80000000u)) ? v[c + 1] : 0.0f;
             dbs[c] += d0;
             dbs[c + 1] += d1;
-            o[k2] = (uint32_t)f2bf(d0) | ((uint32_t)f2bf(d1) << 16);
+            o[k2] = pack_bf2(d0, d1);
           }
-          *(uint4*)(act + g * kPlane + off) = make_uint4(o[0], o[1], o[2], o[3]);
+          *(uint4*)(ap + g * kPlane) = make_uint4(o[0], o[1], o[2], o[3]);
         }
       }
-      for (int c = 0; c < 32; c++) {
-        float s = dbs[c];
-        for (int o2 = 16; o2 > 0; o2 >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o2);
-        if (lane == 0) dbp[warp * 32 + c] = s;
-      }
-      tc_fence_before();
-      __syncthreads();
-      if (t < 32) {
-        float s = 0.0f;
-        for (int w2 = 0; w2 < 8; w2++) s += dbp[w2 * 32 + t];
-        part[layer == 2 ? kOffB1 + t : cnn_off_b(layer - 1) + t] += s;
-      }
-      // next layer: the old dZ_l buffer takes a_{l-2}
-      if (layer > 2) cnn_load_act(dz, A.acts, blk, layer - 3);
+      // a lane ends with channel lane / 2 of its half
+      const float s = warp_sum<16>(dbs, lane);
+      if (!(lane & 1)) dbp[w8 * 32 + hw * 16 + (lane >> 1)] = s;
       uint8_t* tmp = dz;
       dz = act;
       act = tmp;
-      __syncthreads();
     }
     if (!ok) break;
+    __syncthreads();
     // layer 1: dW1[co][input][tap] = sum_p dZ1[p][co] in[p + tap] (dZ1 is in
     // dz; the second input is the constant QP plane, zero in the halo). Warp
-    // w takes rows 4w..4w+3 and lane the output channel, over a sliding 3x3
-    // window of (input, inside) pairs; the 8 row groups' sums meet in the
-    // weight buffer (free until the next block) and are added in a fixed order.
+    // w of a half takes rows 4w..4w+3 and lane the output channel, over a
+    // sliding 3x3 window of the half's input plane; the 8 row groups' sums
+    // meet in shared memory and are added in a fixed order.
     {
       const uint8_t* zp = dz + (lane >> 3) * kPlane + (lane & 7) * 2;
-      float sx[9], sq[9];
+      const uint16_t* xp = (const uint16_t*)xpad + hw;
+      float sx[9];
 #pragma unroll
-      for (int k = 0; k < 9; k++) sx[k] = sq[k] = 0.0f;
-      for (int y = 4 * warp; y < 4 * warp + 4; y++) {
-        float2 w[3][3];
+      for (int k = 0; k < 9; k++) sx[k] = 0.0f;
+#pragma unroll 1
+      for (int y = 4 * w8; y < 4 * w8 + 4; y++) {
+        float w[3][3];
 #pragma unroll
         for (int dy = 0; dy < 3; dy++)
 #pragma unroll
-          for (int dx = 0; dx < 2; dx++) w[dy][dx + 1] = xpad[(y + dy) * 34 + dx];
+          for (int dx = 0; dx < 2; dx++) w[dy][dx + 1] = bf2f(xp[2 * ((y + dy) * 34 + dx)]);
+#pragma unroll 8
         for (int x = 0; x < 32; x++) {
 #pragma unroll
           for (int dy = 0; dy < 3; dy++) {
             w[dy][0] = w[dy][1];
             w[dy][1] = w[dy][2];
-            w[dy][2] = xpad[(y + dy) * 34 + x + 2];
+            w[dy][2] = bf2f(xp[2 * ((y + dy) * 34 + x + 2)]);
           }
           const float z = bf2f(*(const uint16_t*)(zp + ((y + 1) * kImgW + x + 1) * 16));
 #pragma unroll
-          for (int k = 0; k < 9; k++) {
-            sx[k] = fmaf(z, w[k / 3][k % 3].x, sx[k]);
-            sq[k] = fmaf(z, w[k / 3][k % 3].y, sq[k]);
-          }
+          for (int k = 0; k < 9; k++) sx[k] = fmaf(z, w[k / 3][k % 3], sx[k]);
         }
       }
-      float* red = (float*)Wt;  // [8 row groups][32 channels][18]
 #pragma unroll
-      for (int k = 0; k < 9; k++) {
-        red[(warp * 32 + lane) * 18 + k] = sx[k];
-        red[(warp * 32 + lane) * 18 + 9 + k] = sq[k];
+      for (int k = 0; k < 9; k++) red[(w8 * 32 + lane) * 18 + hw * 9 + k] = sx[k];
+      if (warp == 3) {
+        float s = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 8; w++) s += dbp[w * 32 + lane];
+        part[kSlW1 + kOffB1 + lane] += s;
       }
       __syncthreads();
-      for (int o = t; o < 32 * 18; o += kCnnThreads) {
+      for (int o = t; o < 32 * 18; o += kCnnBwdThreads) {
         float v = 0.0f;
+#pragma unroll
         for (int g = 0; g < 8; g++) v += red[g * 32 * 18 + o];
-        part[kOffW1 + o] += (o % 18) < 9 ? v : v * A.qp_in;
+        part[kSlW1 + o] += (o % 18) < 9 ? v : v * A.qp_in;
       }
     }
-    __syncthreads();
+    blk = next;
   }
   if (!ok && t == 0) atomicOr(A.status, 1u);
+  if (ok && pending >= 0) cnn_drain_dw(part, tmem + 256, pending, warp, lane);
+  cnn_load_wait<0>();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, kCnnBwdCols);
 }
 
-// grads[i] = sum over the CTA slices; loss[0] = sum of the loss slots.
+// grads = the sum over the CTA slices in their order, a thread per value of a
+// slice (taps 9 of the last tap pair are no values); loss[0] = that of the
+// loss slots.
 __global__ void k_cnn_reduce(const float* __restrict__ partial, int slices, float* __restrict__ grads,
                              float* __restrict__ loss) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i > kCnnParams) return;
+  if (i > kSlLoss) return;
+  float* dst;
+  if (i < kSlW1) {
+    const int l = i / (5 * 2048), r = i % (5 * 2048), lane = r & 31;
+    const int tap = 2 * (r / 2048) + (lane >> 4), row = 16 * ((r >> 5) & 1) + (lane & 15), col = (r >> 6) & 31;
+    if (tap > 8) return;
+    // the rows are the channels of the image at P: dZ in layers 4 and 2, the activation in layer 3
+    const int co = l == 1 ? col : row, ci = l == 1 ? row : col;
+    dst = grads + cnn_off_w(2 + l) + (co * kCnnCh + ci) * 9 + tap;
+  } else if (i < kSlB) {
+    dst = grads + i - kSlW1;
+  } else if (i < kSlHeads) {
+    dst = grads + cnn_off_b(2 + (i - kSlB) / 32) + (i - kSlB) % 32;
+  } else if (i < kSlLoss) {
+    dst = grads + kOffWi + i - kSlHeads;
+  } else {
+    dst = loss;
+  }
   float s = 0.0f;
-  for (int k = 0; k < slices; k++) s += partial[(size_t)k * (kCnnParams + 1) + i];
-  if (i < kCnnParams)
-    grads[i] = s;
-  else
-    loss[0] = s;
+#pragma unroll 16
+  for (int k = 0; k < slices; k++) s += partial[(size_t)k * kCnnSlice + i];
+  *dst = s;
 }
 
 // Adam (bias-corrected) on the fp32 parameter vector.

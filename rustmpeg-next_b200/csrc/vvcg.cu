@@ -1812,7 +1812,7 @@ static vvcg_status cnn_train_step(vvcg_ctx* ctx, const uint16_t* plane, uint64_t
   CK(ctx->d_cnn_acts.reserve((size_t)num_blocks * 4 * 1024 * 32 * 2), "cudaMalloc");
   CK(ctx->d_cnn_logits.reserve((size_t)num_blocks * kCnnOut * 4), "cudaMalloc");
   CK(ctx->d_cnn_gap.reserve((size_t)num_blocks * 32 * 4), "cudaMalloc");
-  CK(ctx->d_cnn_partial.reserve((size_t)grid * (kCnnParams + 1) * 4), "cudaMalloc");
+  CK(ctx->d_cnn_partial.reserve((size_t)grid * kCnnSlice * 4), "cudaMalloc");
   k_cnn_pack<<<(3 * kCnnConvW + 255) / 256, 256, 0, ctx->stream>>>(params, (uint16_t*)ctx->d_cnn_pack.p, false);
   k_cnn_pack<<<(3 * kCnnConvW + 255) / 256, 256, 0, ctx->stream>>>(params, (uint16_t*)ctx->d_cnn_packT.p, true);
   CK(cudaGetLastError(), "cnn pack launch");
@@ -1826,9 +1826,9 @@ static vvcg_status cnn_train_step(vvcg_ctx* ctx, const uint16_t* plane, uint64_t
                (const float*)ctx->d_cnn_logits.p,
                (const float*)ctx->d_cnn_gap.p, (const uint16_t*)ctx->d_cnn_acts.p, (float*)ctx->d_cnn_partial.p,
                1.0f / (float)num_blocks, status};
-  k_cnn_backward<<<grid, kCnnThreads, kCnnBwdSmem, ctx->stream>>>(B);
+  k_cnn_backward<<<grid, kCnnBwdThreads, kCnnBwdSmem, ctx->stream>>>(B);
   CK(cudaGetLastError(), "cnn backward launch");
-  k_cnn_reduce<<<(kCnnParams + 1 + 255) / 256, 256, 0, ctx->stream>>>((const float*)ctx->d_cnn_partial.p, (int)grid,
+  k_cnn_reduce<<<(kSlLoss + 1 + 127) / 128, 128, 0, ctx->stream>>>((const float*)ctx->d_cnn_partial.p, (int)grid,
                                                                       grads, loss);
   CK(cudaGetLastError(), "cnn reduce launch");
   ctx->launches += 5;
