@@ -453,7 +453,7 @@ namespace vvcg {
 // the activations come by cp.async, the next layer's (or block's) into the
 // buffer that the layer has done with, during its epilogue; a layer's weight
 // gradient is read out of TMEM while the next input gradient's MMAs run.
-// 1024 blocks: 958 -> 447 us, the 432 + 1728 MMAs of a block 62 k of 106 k cycles
+// 1024 blocks: 958 -> 442 us, the 432 + 1728 MMAs of a block 62 k of 106 k cycles
 // at the rate of their operand reads.
 struct CnnBwdArgs {
   const uint16_t* plane;
@@ -552,11 +552,13 @@ __device__ __forceinline__ int cnn_next_block(const CnnBwdArgs& A, int blk) {
 // Adds the weight gradient in TMEM to the slice of layer li: lane quarters 0
 // and 1 hold rows 0..31 (the channels of the image at P), a lane tap
 // 2 g + lane / 16 of row 16 q + lane % 16, a column the other image's channel.
+// kWarps warps, numbered from 0, take part.
+template <int kWarps>
 __device__ __forceinline__ void cnn_drain_dw(float* part, uint32_t tmem, int li, int warp, int lane) {
   const int q = warp & 3;
   if (q >= 2) return;
 #pragma unroll 1
-  for (int u = warp >> 2; u < 10; u += kCnnBwdThreads / 128) {
+  for (int u = warp >> 2; u < 10; u += kWarps / 4) {
     const int g = u >> 1;
     float v[16], o[16];
     tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + u * 16, v);
@@ -605,7 +607,6 @@ __global__ void __launch_bounds__(kCnnBwdThreads, 1) k_cnn_backward(const __grid
   const uint32_t tmem = *tslot;
   uint32_t phase = 0;
   bool ok = true;
-  int pending = -1;  // the layer (minus 2) whose weight gradient is in TMEM
 
   if (blk < A.n) cnn_load_act(P, A.acts, blk, 3);
   while (blk < A.n) {
@@ -728,8 +729,8 @@ __global__ void __launch_bounds__(kCnnBwdThreads, 1) k_cnn_backward(const __grid
       if (warp == 2) {
         if (elect_one()) cnn_issue_layer(tmem, smem_u32(dz), smem_u32(Wt) + li * kPackL, mbar, false);
         __syncwarp();
-      } else if (pending >= 0) {
-        cnn_drain_dw(part, tmem + 256, pending, warp, lane);
+      } else if (layer < 4) {
+        cnn_drain_dw<16>(part, tmem + 256, li + 1, warp, lane);
       }
       if (warp == 3) {  // the bias gradient of this layer
         float s = 0.0f;
@@ -751,7 +752,6 @@ __global__ void __launch_bounds__(kCnnBwdThreads, 1) k_cnn_backward(const __grid
       phase ^= 1;
       tc_fence_after();
       if (!ok) break;
-      pending = li;
       // the old dZ_l buffer takes a_{l-2}, or the next block's a4
       if (layer > 2)
         cnn_load_act(dz, A.acts, blk, layer - 3);
@@ -798,43 +798,59 @@ __global__ void __launch_bounds__(kCnnBwdThreads, 1) k_cnn_backward(const __grid
     __syncthreads();
     // layer 1: dW1[co][input][tap] = sum_p dZ1[p][co] in[p + tap] (dZ1 is in
     // dz; the second input is the constant QP plane, zero in the halo). Warp
-    // w of a half takes rows 4w..4w+3 and lane the output channel, over a
-    // sliding 3x3 window of the half's input plane; the 8 row groups' sums
-    // meet in shared memory and are added in a fixed order.
-    {
-      const uint8_t* zp = dz + (lane >> 3) * kPlane + (lane & 7) * 2;
-      const uint16_t* xp = (const uint16_t*)xpad + hw;
-      float sx[9];
+    // w of the first half takes rows 4w..4w+3, a lane a pair of channels and
+    // one of the two input planes, over a sliding 3x3 window in packed fp32;
+    // the 8 row groups' sums meet in shared memory and are added in a fixed
+    // order. Meanwhile the second half takes layer 2's weight gradient.
+    if (hw == 1) {
+      cnn_drain_dw<8>(part, tmem + 256, 0, warp - 8, lane);
+      if (warp == 11) {
+        float s = 0.0f;
 #pragma unroll
-      for (int k = 0; k < 9; k++) sx[k] = 0.0f;
+        for (int w = 0; w < 8; w++) s += dbp[w * 32 + lane];
+        part[kSlW1 + kOffB1 + lane] += s;
+      }
+      tc_fence_before();
+    } else {
+      const int c2 = lane & 15, in = lane >> 4;
+      const uint8_t* zp = dz + (c2 >> 2) * kPlane + (c2 & 3) * 4;
+      const uint16_t* xp = (const uint16_t*)xpad + in;
+      auto window = [&](int i) {
+        const float f = bf2f(xp[2 * i]);
+        return f2_pack(f, f);
+      };
+      uint64_t sx[9];
+#pragma unroll
+      for (int k = 0; k < 9; k++) sx[k] = 0ull;
 #pragma unroll 1
       for (int y = 4 * w8; y < 4 * w8 + 4; y++) {
-        float w[3][3];
+        uint64_t w[3][3];
 #pragma unroll
         for (int dy = 0; dy < 3; dy++)
 #pragma unroll
-          for (int dx = 0; dx < 2; dx++) w[dy][dx + 1] = bf2f(xp[2 * ((y + dy) * 34 + dx)]);
+          for (int dx = 0; dx < 2; dx++) w[dy][dx + 1] = window((y + dy) * 34 + dx);
 #pragma unroll 8
         for (int x = 0; x < 32; x++) {
 #pragma unroll
           for (int dy = 0; dy < 3; dy++) {
             w[dy][0] = w[dy][1];
             w[dy][1] = w[dy][2];
-            w[dy][2] = bf2f(xp[2 * ((y + dy) * 34 + x + 2)]);
+            w[dy][2] = window((y + dy) * 34 + x + 2);
           }
-          const float z = bf2f(*(const uint16_t*)(zp + ((y + 1) * kImgW + x + 1) * 16));
+          const uint32_t zz = *(const uint32_t*)(zp + ((y + 1) * kImgW + x + 1) * 16);
+          const uint64_t z = f2_pack(__uint_as_float(zz << 16), __uint_as_float(zz & 0xFFFF0000u));
 #pragma unroll
-          for (int k = 0; k < 9; k++) sx[k] = fmaf(z, w[k / 3][k % 3], sx[k]);
+          for (int k = 0; k < 9; k++) sx[k] = f2_fma(z, w[k / 3][k % 3], sx[k]);
         }
       }
 #pragma unroll
-      for (int k = 0; k < 9; k++) red[(w8 * 32 + lane) * 18 + hw * 9 + k] = sx[k];
-      if (warp == 3) {
-        float s = 0.0f;
-#pragma unroll
-        for (int w = 0; w < 8; w++) s += dbp[w * 32 + lane];
-        part[kSlW1 + kOffB1 + lane] += s;
+      for (int k = 0; k < 9; k++) {
+        const float2 v = f2_unpack(sx[k]);
+        red[(w8 * 32 + 2 * c2) * 18 + in * 9 + k] = v.x;
+        red[(w8 * 32 + 2 * c2 + 1) * 18 + in * 9 + k] = v.y;
       }
+    }
+    {
       __syncthreads();
       for (int o = t; o < 32 * 18; o += kCnnBwdThreads) {
         float v = 0.0f;
@@ -846,7 +862,6 @@ __global__ void __launch_bounds__(kCnnBwdThreads, 1) k_cnn_backward(const __grid
     blk = next;
   }
   if (!ok && t == 0) atomicOr(A.status, 1u);
-  if (ok && pending >= 0) cnn_drain_dw(part, tmem + 256, pending, warp, lane);
   cnn_load_wait<0>();
   tc_fence_before();
   __syncthreads();
