@@ -2718,7 +2718,7 @@ extern "C" vvcg_status vvcg_tu_autotune(vvcg_ctx* ctx, const vvcg_tu_rec* recs, 
 // is part of the library's module image: nothing is allocated per call. The
 // residuals go into the caller's planes (DevPic::scratch aliases
 // DevPic::plane): the wavefront kernel reads each sample's residual in the
-// same lane, just before it stores that sample's reconstruction, and
+// thread that stores that sample's reconstruction, before it does, and
 // neighbouring blocks only read samples that are already reconstructed.
 // ---------------------------------------------------------------------------
 namespace {
