@@ -282,9 +282,10 @@ __device__ __forceinline__ void predict_run(int r, const ModeInfo& m, int w, int
   }
 }
 
-// clip(prediction + residual) of a pair of samples: the residual is clamped
-// to +-4096 first, which changes no clipped sum (predictions are at most
-// 4095) and keeps the packed addition inside 16 bits.
+// clip(prediction + residual) of a pair of samples, for predictions of 0..4095
+// (what the intra predictors and 8-bit references give): the residual is
+// clamped to +-4096 first, which changes no clipped sum of such predictions
+// and keeps the packed addition inside 16 bits.
 __device__ __forceinline__ uint32_t add_clip2(uint32_t pred, uint32_t res, uint32_t max2) {
   res = __vmaxs2(__vmins2(res, 0x10001000u), 0xF000F000u);
   return __vmins2(__vmaxs2(__vadd2(pred, res), 0u), max2);

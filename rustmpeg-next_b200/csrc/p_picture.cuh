@@ -101,6 +101,14 @@ __device__ __forceinline__ void p_predict_tile(const PPicDev& P, const vvcg_inte
     p_tile_wide<kLuma>(&P, &P.cus[cu], comp, bx, by, pred);
 }
 
+// clip(prediction + residual) to 8 bits of a pair of 16-bit numbers, in 32
+// bits: whole-sample motion copies reference samples above 8 bits as they
+// are, outside the range in which add_clip2 is exact.
+__device__ __forceinline__ uint32_t p_add_wide2(uint32_t pred, uint32_t res) {
+  const int lo = (int)(int16_t)pred + (int)(int16_t)res, hi = ((int)pred >> 16) + ((int)res >> 16);
+  return (uint32_t)clampi(lo, 0, 255) | (uint32_t)clampi(hi, 0, 255) << 16;
+}
+
 // Grid: (CTUs of the largest picture of the level, pictures of the level).
 // The unit's work is cut into near-equal parts: warp 0 turns the luma levels
 // into the residual, warps 1 and 2 a chroma component's and then predict half
@@ -179,10 +187,13 @@ k_p_cu(const PPicDev* __restrict__ pics, const int16_t* __restrict__ levels, uin
     const int k = comp == 0 ? r : (comp == 1 ? r - 128 : r - 160);
     const int x = comp ? 8 * (k & 1) : 8 * (k & 3), y = comp ? k >> 1 : k >> 2;
     const uint4 p = *reinterpret_cast<const uint4*>(&pred[8 * r]), d = *reinterpret_cast<const uint4*>(&res[8 * r]);
+    uint16_t* const at = P.out[comp] + (size_t)((comp ? by / 2 : by) + y) * P.stride[comp] + (comp ? bx / 2 : bx) + x;
     constexpr uint32_t top = 0x00FF00FFu;
-    *reinterpret_cast<uint4*>(P.out[comp] + (size_t)((comp ? by / 2 : by) + y) * P.stride[comp] + (comp ? bx / 2 : bx) +
-                              x) = make_uint4(add_clip2(p.x, d.x, top), add_clip2(p.y, d.y, top),
-                                              add_clip2(p.z, d.z, top), add_clip2(p.w, d.w, top));
+    const bool wide = ((p.x | p.y | p.z | p.w) & ~top) != 0;
+    *reinterpret_cast<uint4*>(at) =
+        wide ? make_uint4(p_add_wide2(p.x, d.x), p_add_wide2(p.y, d.y), p_add_wide2(p.z, d.z), p_add_wide2(p.w, d.w))
+             : make_uint4(add_clip2(p.x, d.x, top), add_clip2(p.y, d.y, top), add_clip2(p.z, d.z, top),
+                          add_clip2(p.w, d.w, top));
   }
 }
 
