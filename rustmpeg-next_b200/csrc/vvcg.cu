@@ -72,13 +72,13 @@ struct DevBuf {
 struct PinnedBuf {
   void* p = nullptr;
   size_t cap = 0;
-  cudaError_t reserve(size_t bytes) {
+  cudaError_t reserve(size_t bytes, bool grows = true) {
     if (bytes <= cap) return cudaSuccess;
     if (p) cudaFreeHost(p);
     p = nullptr;
     cap = 0;
     size_t want = std::max(bytes, (size_t)4096);
-    want += want / 4;
+    if (grows) want += want / 4;
     cudaError_t e = cudaHostAlloc(&p, want, cudaHostAllocDefault);
     if (e == cudaSuccess) cap = want;
     return e;
@@ -155,6 +155,7 @@ struct vvcg_ctx {
   // rebased records of a pipelined chunk
   PinnedBuf stage, stage_cus;
   PinnedBuf down;  // slots of download_large
+  bool large_down = false;  // a large copy into pageable memory was made
   size_t stage_used = 0;
   GenPass* gen = nullptr;  // state of vvcg_gen_prepare / vvcg_gen_run
   PState* p = nullptr;     // picture buffer and P-picture state (vvcg_dpb_*, vvcg_decode_p_batch)
@@ -2375,13 +2376,20 @@ extern "C" vvcg_status vvcg_encode_sizes(const vvcg_pic_desc* pics, uint32_t num
 // pageable memory goes through pinned slots that several threads empty: the
 // runtime's own path has one thread copy, which also takes the page faults of
 // memory not yet touched (encoding four 1080p pictures into fresh arrays, 25
-// MB of levels: 5.85 ms a call, 4.78 with the slots; 2.95 into pinned memory).
+// MB of levels: 5.95 ms a call, 4.95 with the slots; 2.95 into pinned memory).
 // Each thread keeps two slots in flight; eight threads were slower than four
-// (5.7 ms: they contend for the address space). Pinned, managed and device
-// destinations and copies below kDownMin, where the threads cost more than
-// they save, take one transfer, as does everything when the slots cannot be
-// had. On return a pageable destination is written.
-static constexpr size_t kDownSlot = 1 << 20, kDownMin = 4 << 20;
+// (5.7 ms: they contend for the address space).
+// What they cost: pinning the 8 MB takes 3 to 10 ms once (a first call of four
+// pictures 8.0 to 9.6 ms without, 11 to 21 with), and starting and joining the
+// threads outweighs them in small copies (6 MB: 2.9 -> 3.2 ms a call, 12 MB:
+// 3.95 -> 3.8, 19 MB: 4.93 -> 4.33). So kDownMin lies where the slots gain more
+// than half a millisecond a call, and a context pins them for its second such
+// copy: a program that makes one never pays for them, others have it back
+// after ten calls or so.
+// Pinned, managed and device destinations and smaller copies take one
+// transfer, as does everything when the slots cannot be had. On return a
+// pageable destination is written.
+static constexpr size_t kDownSlot = 1 << 20, kDownMin = 16 << 20;
 static constexpr int kDownThreads = 4;
 
 static bool large_pageable(const void* dst, size_t bytes) {
@@ -2395,7 +2403,11 @@ static bool large_pageable(const void* dst, size_t bytes) {
 static cudaError_t download_large(vvcg_ctx* ctx, void* dst, const void* src, size_t bytes) {
   if (!large_pageable(dst, bytes))
     return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, ctx->stream);
-  if (ctx->down.reserve(2 * kDownThreads * kDownSlot) != cudaSuccess) {
+  if (!ctx->large_down) {
+    ctx->large_down = true;
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, ctx->stream);
+  }
+  if (ctx->down.reserve(2 * kDownThreads * kDownSlot, false) != cudaSuccess) {
     cudaGetLastError();
     return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, ctx->stream);
   }
