@@ -14,7 +14,7 @@
 // progress word.
 //
 // Follows slice::decode_vvc_frame_picture_with_chroma_qp (slice.rs:4834-4988):
-// predict_coded_block_16 / predict_cclm_with_format_16 prediction (intra.cuh),
+// predict_coded_block_16 / predict_cclm_with_format_16 prediction (intra_group.cuh),
 // dequantize_rect_bd or dequantize_dep_quant_bd (dct.rs:1151, :1191),
 // inverse_transform_rect_bd (dct.rs:996) with DCT-II both ways, and the add /
 // clip to 0..2^bd-1. All sums are exact in int32, so reassociating the matrix
@@ -480,8 +480,8 @@ __device__ __forceinline__ void pilot_unit(const DevPic& P, const vvcg_cu_rec& r
 // took 21 us a step; here the 1,536 samples of a unit are spread over 192
 // threads (a run of eight each), a pilot warp prepares the units' modes one
 // step ahead and polls, a publisher warp fences and releases, and the
-// residuals are fetched a step ahead: 3.1 us a step. One 1920x1088 10-bit
-// 4:2:0 picture: 2.41 -> 0.39 ms; 32 of them: 0.74 ms; 128: 5.5 -> 1.9 ms (there
+// residuals are fetched a step ahead: 2.9 us a step. One 1920x1088 10-bit
+// 4:2:0 picture: 2.41 -> 0.37 ms; 32 of them: 0.74 ms; 128: 5.5 -> 1.66 ms (there
 // the CTAs wait at their barriers, 13 of 25 stall cycles an issue).
 template <int kCw>
 __global__ void __launch_bounds__(ReconShape<kCw>::kThreads, ReconShape<kCw>::kCtasPerSm)
@@ -554,28 +554,27 @@ k_recon_rows(const DevPic* __restrict__ pics, const RowItem* __restrict__ rows, 
       ModeRefs& S = W.refs[comp];
       int16_t* tile = W.tile[comp];
       const int w = comp ? P.tb_cw : 32, h = comp ? P.tb_ch : 32, lw = ilog2(max(w, 1));
-      const int nruns = (w * h) >> 3;  // 0 without chroma
+      const bool run = 8 * g.tid < w * h;  // the thread has a run (the variant gives every run one)
       const int st = P.stride[comp], bd = P.bd, cf = P.cf;
       const uint32_t max2 = ((1u << bd) - 1) * 0x10001u;
       uint16_t* const plane = P.plane[comp];
       const int16_t* const scratch = reinterpret_cast<const int16_t*>(P.scratch[comp]);
       const int nref = 2 * (w + h) + 1;
       const int ux = w, uy = h;  // a unit's size in the component's samples
-      auto load_res = [&](const UnitInfo& U, int r) -> uint4 {
-        if (!((U.resid >> comp) & 1)) return make_uint4(0, 0, 0, 0);
-        const int x = 8 * (r & ((w >> 3) - 1)), y = r >> (lw - 3);
+      auto load_res = [&](const UnitInfo& U) -> uint4 {
+        if (!run || !((U.resid >> comp) & 1)) return make_uint4(0, 0, 0, 0);
+        const int x = 8 * (g.tid & ((w >> 3) - 1)), y = g.tid >> (lw - 3);
         return __ldcs(reinterpret_cast<const uint4*>(scratch + (size_t)(U.gy * uy + y) * st + U.gx * ux + x));
       };
       part_sync<4>(kMain + 32);
-      uint4 res = make_uint4(0, 0, 0, 0);
-      if (g.tid < nruns) res = load_res(W.unit[0], g.tid);
+      uint4 res = load_res(W.unit[0]);
       for (int s = 0; s < steps; s++) {
         const UnitInfo& U = W.unit[s & 3];
         const int gx = U.gx, gy = U.gy;
         const int cclm = U.cclm;
         uint16_t* const at = plane + (size_t)(gy * uy) * st + gx * ux;
         RefGeo G{at, st, w, h, 1 << (bd - 1), gy > 0, gx > 0, U.ar != 0, U.bl != 0};
-        const int n = nruns ? nref + (comp == 0 && cclm ? kCclmExtra : 0) : 0;
+        const int n = w ? nref + (comp == 0 && cclm ? kCclmExtra : 0) : 0;  // none without chroma
         int o[3];
         bool ok[3];
 #pragma unroll
@@ -601,26 +600,24 @@ k_recon_rows(const DevPic* __restrict__ pics, const RowItem* __restrict__ rows, 
         CclmModel M{0, 0, 0};
         if (comp && cclm) {
           M = warp_cclm_model(P, gx * 32, gy * 32, w, h, cclm - 1, W.raw[0], W.cclm, R);
-        } else if (nruns) {
+        } else if (w) {
           const ModeInfo m = U.mode[comp];
           group_prep(g.tid, g.n, m, w, h, R, S);
           g.sync();
           const int dc = m.mode == 1 ? warp_dc(R, w, h, (1 << bd) - 1) : 0;
-          for (int r = g.tid; r < nruns; r += g.n) predict_run(r, m, w, h, bd, dc, R, S, tile);
+          if (run) predict_run(g.tid, m, w, h, bd, dc, R, S, tile);
           g.sync();
-          for (int r = g.tid; r < nruns; r += g.n)
-            store_run(at, st, lw, max2, r, r == g.tid ? res : load_res(U, r), tile, cclm != 0);
+          if (run) store_run(at, st, lw, max2, g.tid, res, tile, cclm != 0);
         }
         if (cclm) {
           part_sync<6>(kMain);  // the unit's luma is complete
-          if (comp)
-            for (int r = g.tid; r < nruns; r += g.n) {
-              cclm_run(r, cf, bd, gx, lw, M, W.tile[0], W.raw[0], tile);
-              store_run(at, st, lw, max2, r, r == g.tid ? res : load_res(U, r), tile, false);
-            }
+          if (comp && run) {
+            cclm_run(g.tid, cf, bd, gx, lw, M, W.tile[0], W.raw[0], tile);
+            store_run(at, st, lw, max2, g.tid, res, tile, false);
+          }
         }
         part_sync<5>(kMain + 32);
-        if (s + 1 < steps && g.tid < nruns) res = load_res(W.unit[(s + 1) & 3], g.tid);
+        if (s + 1 < steps) res = load_res(W.unit[(s + 1) & 3]);
       }
     }
   }
