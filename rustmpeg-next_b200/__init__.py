@@ -427,7 +427,12 @@ class GenBatch:
 
 
 class Context:
-    """One libvvcg context: a CUDA device, a stream and the device arena."""
+    """One libvvcg context: a CUDA device, a stream and the device arena.
+
+    The context's own stream does not wait for torch's. Calls on CUDA tensors
+    that synchronise do so before as well (tensors just made or filled by torch)
+    and after (results read through torch); for the asynchronous ones the caller
+    orders the two (set_stream, torch_stream_scope)."""
 
     def __init__(self, device: int = 0, spin_limit: int = 0, reserve_bytes: int = 0):
         L = lib()
@@ -710,6 +715,7 @@ class Context:
         reqs = np.ascontiguousarray(reqs, dtype=TXS_REQ_DTYPE)
         res = torch.zeros(len(reqs) * TXS_RES_DTYPE.itemsize, dtype=torch.uint8, device=pred.device)
         self._keep = reqs
+        torch.cuda.synchronize(pred.device)
         self._check(self._L.vvcg_luma_tx_search_dev(self._h, _ptr(reqs), len(reqs), _ptr(pred), _ptr(src),
                                                     pred.numel(), _ptr(levels), _ptr(samples), levels.numel(),
                                                     _ptr(res)))
@@ -745,6 +751,7 @@ class Context:
         reqs = np.ascontiguousarray(reqs, dtype=MIP_REQ_DTYPE)
         res = torch.zeros(len(reqs) * MIP_RES_DTYPE.itemsize, dtype=torch.uint8, device=refs.device)
         self._keep = reqs
+        torch.cuda.synchronize(refs.device)
         self._check(self._L.vvcg_mip_predict_dev(self._h, _ptr(reqs), len(reqs), _ptr(refs), refs.numel(),
                                                  _ptr(src), _ptr(pred), pred.numel(), _ptr(res)))
         torch.cuda.synchronize(refs.device)
@@ -776,6 +783,7 @@ class Context:
             raise InvalidInput("recon and source planes differ in size")
         out = torch.empty(max(len(reqs), 1) * ISR_RES_DTYPE.itemsize, dtype=torch.uint8, device=recon.device)
         self._keep = reqs
+        torch.cuda.synchronize(recon.device)
         self._check(self._L.vvcg_luma_intra_search_8_dev(self._h, _ptr(recon), recon.stride(0), _ptr(src),
                                                          src.stride(0), w, h, _ptr(reqs), len(reqs), _ptr(out)))
         torch.cuda.synchronize(recon.device)
@@ -793,6 +801,8 @@ class Context:
         dst = out if out is not None else torch.empty(max(len(reqs), 1) * CTU_SEARCH_RES_DTYPE.itemsize,
                                                       dtype=torch.uint8, device=src.device)
         self._keep = reqs
+        if out is None or sync:
+            torch.cuda.synchronize(src.device)
         self._check(self._L.vvcg_ctu_search_dev(self._h, _ptr(src), src.stride(0), w, h, bit_depth, lambda_q8,
                                                 _ptr(reqs), len(reqs), _ptr(dst)))
         if out is not None and not sync:
@@ -815,6 +825,8 @@ class Context:
         acts = torch.empty((n, 4, 1024, 32), dtype=torch.bfloat16, device=dev) if want_acts else None
         st = torch.zeros(1, dtype=torch.int32, device=dev)
         h, w = plane.shape
+        if sync:
+            torch.cuda.synchronize(dev)
         self._check(self._L.vvcg_cnn_forward_dev(self._h, _ptr(plane), plane.stride(0), w, h, bit_depth, qp,
                                                  _ptr(xy.contiguous()), n, _ptr(params), _ptr(logits), _ptr(gap),
                                                  _ptr(acts), _ptr(st)))
@@ -841,6 +853,8 @@ class Context:
         loss = torch.empty(1, dtype=torch.float32, device=dev)
         st = torch.zeros(1, dtype=torch.int32, device=dev)
         h, w = plane.shape
+        if sync:
+            torch.cuda.synchronize(dev)
         if soft is None:
             self._check(self._L.vvcg_cnn_train_step_dev(
                 self._h, _ptr(plane), plane.stride(0), w, h, bit_depth, qp, _ptr(xy.contiguous()),
@@ -870,7 +884,9 @@ class Context:
 
         d = torch.zeros((128, 32), dtype=torch.float32, device=a.device)
         st = torch.zeros(1, dtype=torch.int32, device=a.device)
-        self._check(self._L.vvcg_tc_selftest_dev(self._h, _ptr(a.contiguous()), _ptr(b.contiguous()), _ptr(d),
+        a, b = a.contiguous(), b.contiguous()
+        torch.cuda.synchronize(a.device)
+        self._check(self._L.vvcg_tc_selftest_dev(self._h, _ptr(a), _ptr(b), _ptr(d),
                                                  _ptr(st)))
         torch.cuda.synchronize(a.device)
         if int(st.item()):
@@ -892,6 +908,8 @@ class Context:
         h, w = src.shape
         dst = out if out is not None else torch.empty(max(n, 1) * CTU_SEARCH_RES_DTYPE.itemsize, dtype=torch.uint8,
                                                       device=src.device)
+        if sync:
+            torch.cuda.synchronize(src.device)
         self._check(self._L.vvcg_ctu_search_pruned_rule_dev(
             self._h, _ptr(src), src.stride(0), w, h, bit_depth, lambda_q8, _ptr(xy.contiguous()), n, _ptr(logits),
             top_modes, top_splits, threshold, rule, _ptr(dst)))
@@ -910,6 +928,7 @@ class Context:
         h, w = src.shape
         dst = torch.empty(max(n, 1) * CTU_SEARCH_RES_DTYPE.itemsize, dtype=torch.uint8, device=src.device)
         costs = torch.empty((max(n, 1), 67), dtype=torch.int32, device=src.device)
+        torch.cuda.synchronize(src.device)
         self._check(self._L.vvcg_ctu_search_costs_dev(self._h, _ptr(src), src.stride(0), w, h, bit_depth, lambda_q8,
                                                       _ptr(xy.contiguous()), n, _ptr(dst), _ptr(costs)))
         torch.cuda.synchronize(src.device)
@@ -933,6 +952,7 @@ class Context:
         st.bit_depth, st.vert_collocated, st.ctu_size = bit_depth, int(vert_collocated), ctu
         out = torch.zeros(max(out_count, 1), dtype=torch.int16, device=planes[0].device)
         self._keep = (reqs, st)
+        torch.cuda.synchronize(planes[0].device)
         self._check(self._L.vvcg_gen_intra_predict_dev(self._h, C.byref(st), _ptr(reqs), len(reqs), _ptr(out),
                                                        out_count))
         torch.cuda.synchronize(planes[0].device)
@@ -958,15 +978,13 @@ class Context:
         st.bit_depth, st.vert_collocated, st.ctu_size = bit_depth, int(vert_collocated), ctu
         pred = torch.zeros(max(out_count, 1), dtype=torch.int16, device=planes[0].device)
         self._keep = (reqs, groups, st)
+        torch.cuda.synchronize(planes[0].device)
         self._check(self._L.vvcg_gen_intra_recon_dev(self._h, C.byref(st), _ptr(reqs), len(reqs), _ptr(groups),
                                                      len(groups) - 1, _ptr(residual), _ptr(pred), out_count))
         torch.cuda.synchronize(planes[0].device)
         return pred
 
     # -- inter-prediction tools (device int32 arrays; requests are host records) --
-    # The context's stream does not wait for torch's: each call synchronises
-    # the device before (tensors just made or filled by torch) and after
-    # (results read through torch).
     def _inter_tool(self, fn, reqs, dtype, dev, *args):
         import torch
 
@@ -1072,6 +1090,7 @@ class Context:
         out = torch.zeros(3, dtype=torch.int64, device=ref.device)
         h, w = ref.shape
         fn = self._L.vvcg_plane_metrics_8_dev if ref.element_size() == 1 else self._L.vvcg_plane_metrics_16_dev
+        torch.cuda.synchronize(ref.device)
         self._check(fn(self._h, _ptr(ref), ref.stride(0), _ptr(dist), dist.stride(0), w, h, _ptr(out)))
         torch.cuda.synchronize(ref.device)
         return tuple(int(v) for v in out.cpu())
@@ -1117,6 +1136,7 @@ class Context:
         l0 = (C.c_void_p * max(len(refs_l0), 1))(*[r.data_ptr() for r in refs_l0])
         l1 = (C.c_void_p * max(len(refs_l1), 1))(*[r.data_ptr() for r in refs_l1])
         out = torch.empty(max(len(reqs), 1) * ME_RES_DTYPE.itemsize, dtype=torch.uint8, device=src.device)
+        torch.cuda.synchronize(src.device)
         self._check(self._L.vvcg_inter_search_8_dev(self._h, _ptr(src), src.stride(0), w, h, l0, len(refs_l0), l1,
                                                     len(refs_l1), _ptr(cands) if len(cands) else None, len(cands),
                                                     _ptr(reqs), len(reqs), _ptr(out)))
@@ -1132,6 +1152,7 @@ class Context:
         reqs = np.ascontiguousarray(reqs, dtype=SPLIT_REQ_DTYPE)
         h, w = plane.shape
         out = torch.empty(max(len(reqs), 1), dtype=torch.uint8, device=plane.device)
+        torch.cuda.synchronize(plane.device)
         self._check(self._L.vvcg_qt_mtt_split_dev(self._h, _ptr(plane), plane.stride(0), w, h, bit_depth, _ptr(reqs),
                                                   len(reqs), _ptr(out)))
         torch.cuda.synchronize(plane.device)
