@@ -57,7 +57,8 @@ typedef struct vvcg_config {
   int32_t device;              /* CUDA device ordinal */
   uint32_t flags;              /* reserved, 0 */
   uint64_t reserve_bytes;      /* device arena to reserve up front (0 = grow on demand) */
-  uint32_t spin_limit;         /* wavefront wait limit in polls (0 = library default) */
+  uint32_t spin_limit;         /* limit in polls of a wavefront's row wait and of the general pass's
+                                  level wait (0 = library default) */
   uint32_t reserved;
 } vvcg_config;
 
@@ -1004,12 +1005,18 @@ typedef struct vvcg_gen_batch {
  * memory) and derives the levels and deblocking maps; run enqueues the pass
  * (graph != 0: as one CUDA graph, captured on the first run of the prepared
  * batch); download synchronises and copies the visible planes to out (3 per
- * picture, host, 16-bit samples). vvcg_decode_general_batch does all three. */
+ * picture, host, 16-bit samples). vvcg_decode_general_batch does all three.
+ * All groups are reconstructed by one launch, in which a group waits for its
+ * picture's level before its own. The wait is bounded (vvcg_config.spin_limit):
+ * when one gives up run still returns VVCG_OK, and download (and so
+ * vvcg_decode_general_batch) returns VVCG_TIMEOUT, the planes then being
+ * incomplete; the next run starts anew, and the context stays usable. */
 vvcg_status vvcg_gen_prepare(vvcg_ctx* ctx, const vvcg_gen_batch* b);
 vvcg_status vvcg_gen_run(vvcg_ctx* ctx, uint32_t graph);
 vvcg_status vvcg_gen_download(vvcg_ctx* ctx, const vvcg_plane_out* out);
 vvcg_status vvcg_decode_general_batch(vvcg_ctx* ctx, const vvcg_gen_batch* b, const vvcg_plane_out* out);
-/* Dependency levels of the prepared batch (the intra kernel's launches per run). */
+/* Dependency levels of the prepared batch: the longest chain of groups that
+ * wait for one another (the intra reconstruction is one launch). */
 uint32_t vvcg_gen_levels(const vvcg_ctx* ctx);
 
 /* ---- CABAC parse of strict-profile pictures (host) ------------------------ */

@@ -468,7 +468,7 @@ struct CnnBwdArgs {
   const float* logits;
   const float* gap;
   const uint16_t* acts;
-  float* partial;  // [gridDim.x][kCnnParams + 1]: gradients, then the loss sum
+  float* partial;  // [gridDim.x][kCnnSlice]: each CTA's slice of gradients and loss (kSl*)
   float inv_batch;
   uint32_t* status;
 };

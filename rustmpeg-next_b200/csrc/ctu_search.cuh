@@ -17,7 +17,7 @@
 // Planar and DC, bit depths above 10 and sources above their bit depth take a
 // lane per line with 32-bit arithmetic.
 //
-// 1,980 CTUs at 10 bits take 1.06 ms, bound by instruction issue (0.6 a cycle and
+// 1,980 CTUs at 10 bits take 1.07 ms, bound by instruction issue (0.6 a cycle and
 // scheduler, 62,000 warp instructions a CTA). With a warp per candidate, one
 // prediction at a time into shared memory and a 16-bit Hadamard from there they
 // took 3.41 ms; with the tile's eight lines unrolled and tasks tile by tile

@@ -477,12 +477,12 @@ __device__ __forceinline__ void pilot_unit(const DevPic& P, const vvcg_cu_rec& r
 // CTU x + 1 of the row above is done, so a picture of W x H CTUs takes at
 // least W + 2 (H - 1) steps, each a poll, one gather round trip, the
 // prediction, the stores and the release of the progress word. A warp per row
-// took 21 us a step; here the 1,536 samples of a unit are spread over 192
+// took 19 us a step; here the 1,536 samples of a unit are spread over 192
 // threads (a run of eight each), a pilot warp prepares the units' modes one
 // step ahead and polls, a publisher warp fences and releases, and the
 // residuals are fetched a step ahead: 2.9 us a step. One 1920x1088 10-bit
 // 4:2:0 picture: 2.41 -> 0.37 ms; 32 of them: 0.74 ms; 128: 5.5 -> 1.66 ms (there
-// the CTAs wait at their barriers, 13 of 25 stall cycles an issue).
+// the CTAs wait at their barriers, 14 of 25 stall cycles an issue).
 template <int kCw>
 __global__ void __launch_bounds__(ReconShape<kCw>::kThreads, ReconShape<kCw>::kCtasPerSm)
 k_recon_rows(const DevPic* __restrict__ pics, const RowItem* __restrict__ rows, uint32_t n_rows,

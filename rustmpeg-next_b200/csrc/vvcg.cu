@@ -858,8 +858,7 @@ vvcg_status enqueue_run(vvcg_ctx* ctx, uint32_t mask, uint32_t epoch, bool clear
     const uint32_t n = (uint32_t)ctx->items.size();
     // The picture with the most chroma decides: of 31 4:2:0 pictures of
     // 1920x1088 and a 4:4:4 one the stage takes 0.79 ms, of 32 4:2:0 ones 0.76
-    // (854x480, 63 and one: 0.328 against 0.321). A launch per format would
-    // cost a queue and a launch and leave the chip to the longer one's tail.
+    // (854x480, 63 and one: 0.328 against 0.321).
     int v = 0;
     for (auto& P : ctx->pics) v = std::max(v, recon_variant(P));
     const uint32_t grid = std::min<uint32_t>(n, (uint32_t)(ctx->num_sms * std::max(1, ctx->recon_per_sm[v])));
